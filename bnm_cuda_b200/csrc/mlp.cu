@@ -3,25 +3,53 @@
 // oversampled CMA-ES candidates can be pre-screened before simulation.
 //
 // Network: in -> [hidden, ReLU] x layers -> out, weights kept in FP32 (master
-// copy for Adam) and rounded to BF16 for the forward GEMMs; activations are
-// stored in BF16; every GEMM accumulates in FP32.  Training (MSE loss, Adam)
-// runs entirely on the device with this file's kernels:
-//   gemm_bf16_kernel  C = A B (+bias, ReLU) on mma.sync m16n8k16 BF16 tensor
-//                     cores with FP32 accumulation; operands are read through
-//                     strides (so W, W^T and X^T need no copies) and A may be
-//                     multiplied by a ReLU mask (the backward of the ReLU fused
-//                     into the dX and dW GEMMs);
-//   bias_grad_kernel, mse_grad_kernel, adam_kernel, cast kernels.
+// copy for Adam) and rounded to BF16 for the GEMMs; activations are stored in
+// BF16; every GEMM accumulates in FP32 (mma.sync m16n8k16).  Training (MSE
+// loss, Adam) runs entirely on the device.
+//
+//   mlp_step_kernel     any number of training steps (forward, loss, backward,
+//                       Adam) in one launch of one thread-block cluster; also
+//                       one step's loss and gradients, and the forward pass of
+//                       networks too wide for the kernel below
+//   mlp_predict_kernel  forward pass, 16 rows per CTA, activations in shared
+//                       memory
+//
+// A step of the surrogate is small (B = 64, 256 wide: 78 MFLOP) and a chain of
+// 2 L dependent GEMMs, so it is bound by latency: of launches, of the loads in
+// front of each GEMM and of the K loop.  One kernel per GEMM took 574 us a step
+// (24 launches, GEMM grids of 4 CTAs at 12-108 us each: one 64 x 64 tile per
+// CTA, element-wise strided loads and two block barriers per 32 K).  Here the
+// phases of a step are separated by the cluster's hardware barrier, and every
+// operand is kept in the order in which the MMA's lanes hold it, in both
+// orientations where two GEMMs need it, padded with zeros to multiples of 16:
+//   A blocks  16 rows x 16 K as uint4 [lane]   (the four A registers)
+//   B blocks   8 rows x 16 K as uint2 [lane]   (the two B registers)
+// so a K step of a 16 x 8 output tile is one 16-byte and one 8-byte coalesced
+// load per lane (as rows, the same step touched eight cache lines a load:
+// 145 us a step), all K steps of a 256-wide layer are in flight at once, a
+// warp's tiles come in twos that share an operand (one tile at a time behind a
+// function call: 100 us a step), and an epilogue writes the next
+// GEMM's operand from its accumulators' own lanes, transposed by movmatrix
+// where the other orientation is wanted.  FP32 weights and Adam's moments are
+// kept in accumulator order too ([tile][lane] float4), and Adam runs in the
+// epilogue of the dW tiles; a layer's weights are updated one phase after the
+// last GEMM that reads them.  The K order of every output's MMAs is ascending
+// in steps of 16 and the other sums are in index order, whatever the cluster
+// size and the tiling.  Measured (19-4x256-4, 2000 rows, batch 64, 4 epochs,
+// parameters set and read back): 71.3 -> 6.2 ms; about 40 us of a step's 42
+// are its 10 phases' load and barrier latencies and Adam.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <random>
+#include <type_traits>
 #include <vector>
 
 #include <cuda_bf16.h>
 
 #include "../../include/bnm_b200.h"
+#include "cluster_util.cuh"
 #include "kernels.h"
 
 int bnm_fail_cuda(cudaError_t e, const char* expr, const char* file, int line);
@@ -29,219 +57,716 @@ int bnm_fail_msg(int code, const char* msg);
 
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 32, SPAD = 8;  // CTA tile and shared-memory row padding
+using bnm::cluster_rank;
+using bnm::cluster_size;
+using bnm::cluster_sync;
+typedef __nv_bfloat16 bf16;
 
-struct GemmOp {
-    int M, N, K;
-    const void* A;       // A(m,k) = A[m*sam + k*sak]
-    long long sam, sak;
-    int a_f32;           // A element type: 1 = float, 0 = bf16
-    const __nv_bfloat16* mask;  // optional: A(m,k) *= (mask[m*smm + k*smk] > 0)
-    long long smm, smk;
-    const void* B;       // B(k,n) = B[k*sbk + n*sbn]
-    long long sbk, sbn;
-    int b_f32;
-    const float* bias;   // optional, [N]
-    int relu;            // epilogue ReLU
-    void* C;             // C[m*ldc + n]
-    long long ldc;
-    int c_f32;           // 1: float output, 0: bf16 output
-    float alpha;
+// A layer on the device.  dinp, doutp: din, dout rounded up to 16.
+struct MlpLayer {
+    int din, dout, dinp, doutp;
+    long long woff, boff;  // W and b in the caller's flat parameter vector
+    long long tile, bias;  // W's tiles (16 o x 8 i; units of one tile) and b in the device's FP32 arrays
+    uint2 *w, *wt;         // BF16 weights as B blocks: n = output, k = input; and n = input, k = output
+    uint4* x;              // input activations as A blocks, k = input (first layer: two sets, by step parity)
+    uint2* xt;             // ... as B blocks, n = input, k = batch row (likewise)
+    float* dz;             // gradient at the layer's output, behind its ReLU mask [batch][doutp]
+    uint4 *dzh, *dzt;      // the same rounded, as A blocks: k = output; and m = output, k = batch row
 };
 
-__device__ __forceinline__ float load_elem(const void* p, long long i, int f32) {
-    return f32 ? static_cast<const float*>(p)[i] : __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
+enum { kTrain = 0, kGrads = 1, kForward = 2 };
+
+struct StepArgs {
+    const MlpLayer* layers;
+    int L, in, out;
+    int mode, steps, batch;
+    float4 *w, *m, *v;     // weights and Adam moments, [tile][lane] in accumulator order
+    float *bw, *bm, *bv;   // biases
+    float* g;              // flat gradient (kGrads)
+    const float *X, *T;    // [.][in], [.][out]
+    const int* idx;        // [steps][batch] rows of X and T, or null: row b
+    const float2* c12;     // [steps] Adam bias corrections
+    float lr, b1, b2, eps;
+    size_t x0, xt0;        // elements of one set of the first layer's x and xt
+    float* tgt;            // [2][batch][out]: targets of the step's rows, by step parity
+    float *yout, *loss;    // [batch][out]; [steps]
+};
+
+__device__ __forceinline__ uint32_t pack2(float x, float y) {
+    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x)) |
+           ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(y)) << 16);
 }
 
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+// 8 x 8 BF16 transpose across the warp: lane (g, t) holds row g, columns 2t, 2t + 1
+__device__ __forceinline__ uint32_t transpose8(uint32_t x) {
+    uint32_t y;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
+}
+
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint4& a, const uint2& b) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
         "{%0,%1,%2,%3};\n"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y));
 }
 
-// 4 warps, each a 32x32 piece of the 64x64 CTA tile: 2 (m16) x 4 (n8) mma tiles.
-__global__ void __launch_bounds__(128) gemm_bf16_kernel(GemmOp op) {
-    __shared__ __align__(16) __nv_bfloat16 As[TM][TK + SPAD];  // [m][k]
-    __shared__ __align__(16) __nv_bfloat16 Bs[TN][TK + SPAD];  // [n][k]
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-    const int g = lane >> 2, t = lane & 3;
-    float acc[2][4][4];
+// Output tiles of 16 x 8: kb MMAs each in ascending K, kFly K blocks in flight
+// ahead of their MMAs (the rest of kb in halving groups, so that no load is
+// predicated).  load(k, a, b): this lane's registers of K block k, nA A blocks
+// times nB B blocks.
+template <int kFly, int nA, int nB, class F>
+__device__ __forceinline__ void mma_group(int k0, float (&d)[nA * nB][4], F load) {
+    uint4 a[kFly][nA];
+    uint2 b[kFly][nB];
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int s = 0; s < kFly; s++) load(k0 + s, a[s], b[s]);
 #pragma unroll
-        for (int jn = 0; jn < 4; jn++)
+    for (int s = 0; s < kFly; s++)
 #pragma unroll
-            for (int q = 0; q < 4; q++) acc[i][jn][q] = 0.f;
-
-    for (int k0 = 0; k0 < op.K; k0 += TK) {
-        for (int e = threadIdx.x; e < TM * TK; e += blockDim.x) {
-            const int r = e / TK, c = e % TK, m = m0 + r, k = k0 + c;
-            float va = 0.f;
-            if (m < op.M && k < op.K) {
-                va = load_elem(op.A, m * op.sam + k * op.sak, op.a_f32);
-                if (op.mask && !(__bfloat162float(op.mask[m * op.smm + k * op.smk]) > 0.f)) va = 0.f;
-            }
-            As[r][c] = __float2bfloat16_rn(va);
-        }
-        for (int e = threadIdx.x; e < TN * TK; e += blockDim.x) {
-            const int r = e / TK, c = e % TK, n = n0 + r, k = k0 + c;
-            const float vb = (n < op.N && k < op.K) ? load_elem(op.B, k * op.sbk + n * op.sbn, op.b_f32) : 0.f;
-            Bs[r][c] = __float2bfloat16_rn(vb);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < TK; kk += 16) {
-            uint32_t af[2][4], bf[4][2];
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const int r = wm + i * 16 + g;
-                af[i][0] = *reinterpret_cast<const uint32_t*>(&As[r][kk + 2 * t]);
-                af[i][1] = *reinterpret_cast<const uint32_t*>(&As[r + 8][kk + 2 * t]);
-                af[i][2] = *reinterpret_cast<const uint32_t*>(&As[r][kk + 2 * t + 8]);
-                af[i][3] = *reinterpret_cast<const uint32_t*>(&As[r + 8][kk + 2 * t + 8]);
-            }
-#pragma unroll
-            for (int jn = 0; jn < 4; jn++) {
-                const int c = wn + jn * 8 + g;
-                bf[jn][0] = *reinterpret_cast<const uint32_t*>(&Bs[c][kk + 2 * t]);
-                bf[jn][1] = *reinterpret_cast<const uint32_t*>(&Bs[c][kk + 2 * t + 8]);
-            }
-#pragma unroll
-            for (int i = 0; i < 2; i++)
-#pragma unroll
-                for (int jn = 0; jn < 4; jn++) mma_bf16(acc[i][jn], af[i], bf[jn]);
-        }
-        __syncthreads();
+        for (int i = 0; i < nA * nB; i++) mma_bf16(d[i], a[s][i / nB], b[s][i % nB]);
+}
+template <int kFly, int nA, int nB, class F>
+__device__ __forceinline__ void mma_rest(int k0, int kb, float (&d)[nA * nB][4], F load) {
+    if (k0 + kFly <= kb) {
+        mma_group<kFly, nA, nB>(k0, d, load);
+        k0 += kFly;
     }
+    if constexpr (kFly > 1) mma_rest<kFly / 2, nA, nB>(k0, kb, d, load);
+}
+template <int kFly, int nA, int nB, class F>
+__device__ __forceinline__ void mma_tiles(int kb, float (&d)[nA * nB][4], F load) {
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+    for (int i = 0; i < nA * nB; i++) d[i][0] = d[i][1] = d[i][2] = d[i][3] = 0.f;
+    int k0 = 0;
+#pragma unroll 1
+    for (; k0 + kFly <= kb; k0 += kFly) mma_group<kFly, nA, nB>(k0, d, load);
+    if constexpr (kFly > 1) mma_rest<kFly / 2, nA, nB>(k0, kb, d, load);
+}
+
+// Adam's update of nP parameters (w, first moment m, second moment v; g the
+// gradients).  The update is the FP32 expression
+//     w - lr (m / c1) / (sqrt(v / c2) + eps)
+// with every operation rounded to nearest.  The hardware has no FP32 division
+// or square root: CUDA's are subroutines with a branch each, which a warp goes
+// through one after the other (about 6000 cycles for the 8 parameters of a
+// lane).  Here the quotients and the root are formed in FP64 to a relative
+// error below 2^-51 and rounded to FP32, without branches, so the parameters'
+// chains interleave.  That gives the same FP32 values: a quotient of two
+// 24-bit numbers, or the root of one, is at least 2^-49 away (relative) from
+// the midpoint of two FP32 neighbours, unless the result is subnormal; lanes
+// with a value near those ranges take the plain expression.
+__device__ __forceinline__ float adam_plain(float w, float m, float v, const StepArgs& a, float c1, float c2) {
+    return w - a.lr * (m / c1) / (sqrtf(v / c2) + a.eps);
+}
+template <int nP>
+__device__ __forceinline__ void adam(const float (&g)[nP], float (&w)[nP], float (&m)[nP], float (&v)[nP],
+                                     const StepArgs& a, float2 c12, double rc1, double rc2) {
+    float nw[nP];
+    bool ok = true;
+    auto safe = [](float x, float lo) { return x == 0.f || (fabsf(x) > lo && fabsf(x) < 1e27f); };
 #pragma unroll
-        for (int jn = 0; jn < 4; jn++)
+    for (int i = 0; i < nP; i++) {
+        m[i] = fmaf(1.f - a.b1, g[i], a.b1 * m[i]);
+        v[i] = fmaf((1.f - a.b2) * g[i], g[i], a.b2 * v[i]);
+        const float mh = (float)((double)m[i] * rc1), vh = (float)((double)v[i] * rc2);
+        // root: two Newton steps on g ~ sqrt(x) with the slope of the first estimate
+        float y;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(vh));
+        const double x = vh, h = 0.5 * (double)y;
+        double r = x * (double)y;
+        r = fma(fma(-r, r, x), h, r);
+        r = fma(fma(-r, r, x), h, r);
+        const float den = (vh == 0.f ? 0.f : (float)r) + a.eps, num = a.lr * mh;
+        // quotient: one Newton step on the reciprocal, one on the quotient
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(den));
+        const double d = den, nd = num;
+        double q = y;
+        q = fma(fma(-d, q, 1.0), q, q);
+        const double q0 = nd * q;
+        nw[i] = w[i] - (float)fma(fma(-d, q0, nd), q, q0);
+        ok = ok && safe(m[i], 1e-27f) && safe(v[i], 1e-27f) && safe(num, 1e-18f) && den > 1e-18f && den < 1e18f;
+    }
+    if (!ok)
+#pragma unroll
+        for (int i = 0; i < nP; i++) nw[i] = adam_plain(w[i], m[i], v[i], a, c12.x, c12.y);
+#pragma unroll
+    for (int i = 0; i < nP; i++) w[i] = nw[i];
+}
+
+constexpr int kStepThreads = 512, kStepWarps = kStepThreads / 32;
+constexpr int kPredThreads = 512, kPredWarps = kPredThreads / 32;
+constexpr int kSmemLayers = 128;  // layer descriptors kept in shared memory (more are read from L1)
+
+// What a step's tile functions share.
+struct Step {
+    const StepArgs& a;
+    const MlpLayer* lay;
+    int par;         // step parity
+    float2 c12;
+    double rc1, rc2; // reciprocals of c12
+    int mt;          // blocks of 16 batch rows
+
+    __device__ const uint4* x(int l) const { return lay[l].x + (l == 0 && par ? a.x0 : 0); }
+    __device__ const uint2* xt(int l) const { return lay[l].xt + (l == 0 && par ? a.xt0 : 0); }
+    __device__ float* tgt() const { return a.tgt + (size_t)par * a.batch * a.out; }
+};
+
+// The rows of X that step `step` uses, rounded, as the first layer's operands
+// (block mb of 16 rows, block k of 16 columns); and their targets (32 values a
+// task).  Done while the step before ends: the gathers are chains of loads.
+__device__ __forceinline__ void gather_x(const Step& st, int step, int mb, int k) {
+    const StepArgs& a = st.a;
+    const int lane = threadIdx.x & 31, c = 16 * k + 2 * (lane & 3), B = a.batch, kb = st.lay[0].dinp / 16;
+    uint32_t v[4];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int m = 16 * mb + (lane >> 2) + 8 * h;
+        const float* p = m < B ? a.X + (size_t)(a.idx ? a.idx[(size_t)step * B + m] : m) * a.in : nullptr;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int i = c + 8 * q;
+            v[h + 2 * q] = pack2(p && i < a.in ? p[i] : 0.f, p && i + 1 < a.in ? p[i + 1] : 0.f);
+        }
+    }
+    uint4* x = st.lay[0].x + (step & 1 ? a.x0 : 0);
+    uint2* xt = st.lay[0].xt + (step & 1 ? a.xt0 : 0) + lane;
+    x[(size_t)(mb * kb + k) * 32 + lane] = make_uint4(v[0], v[1], v[2], v[3]);
+    xt[(size_t)(2 * k * st.mt + mb) * 32] = make_uint2(transpose8(v[0]), transpose8(v[1]));
+    xt[(size_t)((2 * k + 1) * st.mt + mb) * 32] = make_uint2(transpose8(v[2]), transpose8(v[3]));
+}
+__device__ __forceinline__ void gather_t(const StepArgs& a, int step, int task) {
+    const int e = 32 * task + (threadIdx.x & 31), n = a.batch * a.out;
+    if (e >= n) return;
+    const int b = e / a.out;
+    const int r = a.idx ? a.idx[(size_t)step * a.batch + b] : b;
+    a.tgt[(size_t)(step & 1) * n + e] = a.T[(size_t)r * a.out + e % a.out];
+}
+
+// Writes the gradient e of a 16 x 8 tile (rows 16 mb .., columns 8 nb ..) at
+// the output of layer z: FP32, and rounded in both orientations.
+__device__ __forceinline__ void store_dz(const Step& st, const MlpLayer& z, int mb, int nb, const float (&e)[4]) {
+    const int lane = threadIdx.x & 31, m = 16 * mb + (lane >> 2), n = 8 * nb + 2 * (lane & 3), B = st.a.batch;
+    if (m < B) *reinterpret_cast<float2*>(z.dz + (size_t)m * z.doutp + n) = make_float2(e[0], e[1]);
+    if (m + 8 < B) *reinterpret_cast<float2*>(z.dz + (size_t)(m + 8) * z.doutp + n) = make_float2(e[2], e[3]);
+    const uint32_t p0 = pack2(e[0], e[1]), p1 = pack2(e[2], e[3]);
+    // columns 8 nb .. are registers 0, 1 or 2, 3 of A block nb / 2
+    reinterpret_cast<uint2*>(z.dzh + ((size_t)mb * (z.doutp / 16) + nb / 2) * 32 + lane)[nb & 1] = make_uint2(p0, p1);
+    uint32_t* zt = reinterpret_cast<uint32_t*>(z.dzt + ((size_t)(nb / 2) * st.mt + mb) * 32 + lane) + (nb & 1);
+    zt[0] = transpose8(p0);
+    zt[2] = transpose8(p1);
+}
+
+// Forward of layer l, 8 outputs of nA blocks of 16 rows; the last layer also
+// forms the gradient of the MSE at its output.
+template <int nA>
+__device__ __forceinline__ void forward_tiles(const Step& st, int l, int mb, int nb) {
+    const StepArgs& a = st.a;
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, B = a.batch;
+    const MlpLayer& y = st.lay[l];
+    const int n = 8 * nb + 2 * t, kb = y.dinp / 16;
+    const float2 bias = *reinterpret_cast<const float2*>(a.bw + y.bias + n);
+    const uint2* wp = y.w + (size_t)nb * kb * 32 + lane;
+    const uint4* xp = st.x(l) + (size_t)mb * kb * 32 + lane;
+    float d[nA][4];
+    mma_tiles<8, nA, 1>(kb, d, [&](int k, uint4 (&fa)[nA], uint2 (&fb)[1]) {
+#pragma unroll
+        for (int i = 0; i < nA; i++) fa[i] = xp[32 * (i * kb + k)];
+        fb[0] = wp[32 * k];
+    });
+#pragma unroll
+    for (int i = 0; i < nA; i++) {
+        const int m = 16 * (mb + i) + g;
+        const float v[4] = {d[i][0] + bias.x, d[i][1] + bias.y, d[i][2] + bias.x, d[i][3] + bias.y};
+        if (l < a.L - 1) {  // rows past the batch and columns past the layer are zero
+            const MlpLayer& z = st.lay[l + 1];
+            const uint32_t p0 = m < B ? pack2(fmaxf(v[0], 0.f), fmaxf(v[1], 0.f)) : 0u;
+            const uint32_t p1 = m + 8 < B ? pack2(fmaxf(v[2], 0.f), fmaxf(v[3], 0.f)) : 0u;
+            reinterpret_cast<uint2*>(z.x + ((size_t)(mb + i) * (z.dinp / 16) + nb / 2) * 32 + lane)[nb & 1] =
+                make_uint2(p0, p1);
+            if (a.mode != kForward)
+                z.xt[((size_t)nb * st.mt + mb + i) * 32 + lane] = make_uint2(transpose8(p0), transpose8(p1));
+            continue;
+        }
+        float e[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int r = m + 8 * (q >> 1), c = n + (q & 1);
+            e[q] = 0.f;
+            if (r < B && c < a.out) {
+                a.yout[(size_t)r * a.out + c] = v[q];
+                if (a.mode != kForward) {  // MSE: d loss / dy = 2 (y - t) / (B out)
+                    const float df = v[q] - st.tgt()[(size_t)r * a.out + c];
+                    e[q] = 2.f * df / (float)(B * a.out);
+                }
+            }
+        }
+        if (a.mode != kForward) store_dz(st, y, mb + i, nb, e);
+    }
+}
+
+// dX of layer l, 8 inputs of nA blocks of 16 rows: the gradient at the output
+// of layer l - 1, behind its ReLU.
+template <int nA>
+__device__ __forceinline__ void dx_tiles(const Step& st, int l, int mb, int nb) {
+    const int lane = threadIdx.x & 31;
+    const MlpLayer& y = st.lay[l];
+    const int kb = y.doutp / 16;
+    const uint4* ap = y.dzh + (size_t)mb * kb * 32 + lane;
+    const uint2* bp = y.wt + (size_t)nb * kb * 32 + lane;
+    // the activations behind the mask sit in this lane's own registers of the A block
+    uint2 act[nA];
+#pragma unroll
+    for (int i = 0; i < nA; i++)
+        act[i] = reinterpret_cast<const uint2*>(st.x(l) + ((size_t)(mb + i) * (y.dinp / 16) + nb / 2) * 32 + lane)[nb & 1];
+    float d[nA][4];
+    mma_tiles<8, nA, 1>(kb, d, [&](int k, uint4 (&fa)[nA], uint2 (&fb)[1]) {
+#pragma unroll
+        for (int i = 0; i < nA; i++) fa[i] = ap[32 * (i * kb + k)];
+        fb[0] = bp[32 * k];
+    });
+#pragma unroll
+    for (int i = 0; i < nA; i++) {
+        float e[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint32_t xb = q < 2 ? act[i].x : act[i].y;
+            const float x = __uint_as_float((q & 1) ? xb & 0xffff0000u : xb << 16);
+            e[q] = x > 0.f ? d[i][q] : 0.f;  // rows past the batch have x = 0
+        }
+        store_dz(st, st.lay[l - 1], mb + i, nb, e);
+    }
+}
+
+// Bias gradients of 32 outputs: sums over the batch in order.
+__device__ __forceinline__ void db_task(const Step& st, int l, int task) {
+    const StepArgs& a = st.a;
+    const MlpLayer& y = st.lay[l];
+    const int o = task * 32 + (threadIdx.x & 31), B = a.batch, ld = y.doutp;
+    if (o >= y.dout) return;
+    const float* dz = y.dz + o;
+    float s = 0.f;
+    int b = 0;
+    for (; b + 16 <= B; b += 16) {
+        float e[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) e[k] = dz[(size_t)(b + k) * ld];
+#pragma unroll
+        for (int k = 0; k < 16; k++) s += e[k];
+    }
+    for (; b < B; b++) s += dz[(size_t)b * ld];
+    if (a.mode == kGrads) {
+        a.g[y.boff + o] = s;
+        return;
+    }
+    const long long i = y.bias + o;
+    float gi[1] = {s}, wi[1] = {a.bw[i]}, mi[1] = {a.bm[i]}, vi[1] = {a.bv[i]};
+    adam(gi, wi, mi, vi, a, st.c12, st.rc1, st.rc2);
+    a.bm[i] = mi[0];
+    a.bv[i] = vi[0];
+    a.bw[i] = wi[0];
+}
+
+// dW of layer l, 16 outputs o x 16 inputs i (two tiles), K = batch, and Adam's
+// update of its weights; the tasks past the tiles are the biases'.
+__device__ __forceinline__ void dw_task(const Step& st, int l, int task) {
+    const StepArgs& a = st.a;
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const MlpLayer& y = st.lay[l];
+    const int ot = y.doutp / 16, ki = y.dinp / 16;
+    if (task >= ot * ki) {
+        db_task(st, l, task - ot * ki);
+        return;
+    }
+    const int ob = task % ot, ib = 2 * (task / ot), kb = st.mt;
+    const bool train = a.mode == kTrain;
+    const size_t e = (size_t)(y.tile + ib * ot + ob) * 32 + lane;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 wv[2], mv[2], vv[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {  // the parameters' loads overlap the MMAs
+        const size_t ei = e + (size_t)i * ot * 32;
+        wv[i] = train ? a.w[ei] : zero;
+        mv[i] = train ? a.m[ei] : zero;
+        vv[i] = train ? a.v[ei] : zero;
+    }
+    const uint4* ap = y.dzt + (size_t)ob * kb * 32 + lane;
+    float d[2][4];
+    const uint2* bp = st.xt(l) + (size_t)ib * kb * 32 + lane;
+    mma_tiles<4, 1, 2>(kb, d, [&](int k, uint4 (&fa)[1], uint2 (&fb)[2]) {
+        fa[0] = ap[32 * k];
+        fb[0] = bp[32 * k];
+        fb[1] = bp[32 * (kb + k)];
+    });
+    auto inside = [&](int i, int q) {  // accumulator q of tile i is a weight, not padding
+        return 16 * ob + g + 8 * (q >> 1) < y.dout && 8 * (ib + i) + 2 * t + (q & 1) < y.din;
+    };
+    if (!train) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const int i = k >> 2, q = k & 3, o = 16 * ob + g + 8 * (q >> 1), c = 8 * (ib + i) + 2 * t + (q & 1);
+            if (inside(i, q)) a.g[y.woff + (long long)o * y.din + c] = d[i][q];
+        }
+        return;
+    }
+    const float gr[8] = {d[0][0], d[0][1], d[0][2], d[0][3], d[1][0], d[1][1], d[1][2], d[1][3]};
+    float w[8] = {wv[0].x, wv[0].y, wv[0].z, wv[0].w, wv[1].x, wv[1].y, wv[1].z, wv[1].w};
+    float m[8] = {mv[0].x, mv[0].y, mv[0].z, mv[0].w, mv[1].x, mv[1].y, mv[1].z, mv[1].w};
+    float v[8] = {vv[0].x, vv[0].y, vv[0].z, vv[0].w, vv[1].x, vv[1].y, vv[1].z, vv[1].w};
+    adam(gr, w, m, v, a, st.c12, st.rc1, st.rc2);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (!inside(i, q)) w[4 * i + q] = m[4 * i + q] = v[4 * i + q] = 0.f;  // the padding stays zero
+        const size_t ei = e + (size_t)i * ot * 32;
+        a.w[ei] = make_float4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+        a.m[ei] = make_float4(m[4 * i], m[4 * i + 1], m[4 * i + 2], m[4 * i + 3]);
+        a.v[ei] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        const uint32_t p0 = pack2(w[4 * i], w[4 * i + 1]), p1 = pack2(w[4 * i + 2], w[4 * i + 3]);
+        uint32_t* wp = reinterpret_cast<uint32_t*>(y.w + ((size_t)(2 * ob) * ki + ib / 2) * 32 + lane) + i;
+        wp[0] = p0;
+        wp[(size_t)ki * 64] = p1;  // the next 8 outputs' block
+        y.wt[((size_t)(ib + i) * ot + ob) * 32 + lane] = make_uint2(transpose8(p0), transpose8(p1));
+    }
+}
+
+// One cluster; CTA c of it takes the c-th share of a phase's tiles, a warp per
+// tile.  Phases of a step, each ending in a cluster barrier:
+//   forward of layer 0 .. L-1 (the last also forms the output gradient);
+//   for l = L-1 .. 1: dX of layer l, with dW / db (and Adam) of layer l + 1;
+//   dW / db of layers 1 and 0, and the next step's rows of X and T.
+__global__ void __launch_bounds__(kStepThreads, 1) mlp_step_kernel(StepArgs args) {
+    __shared__ float red[256];
+    __shared__ MlpLayer s_lay[kSmemLayers];
+    const int warp = threadIdx.x >> 5;
+    const int nc = (int)cluster_size(), c = (int)cluster_rank();
+    const int L = args.L, B = args.batch;
+    if (L <= kSmemLayers)
+        for (int e = threadIdx.x; e < L * (int)sizeof(MlpLayer) / 4; e += kStepThreads)
+            reinterpret_cast<uint32_t*>(s_lay)[e] = reinterpret_cast<const uint32_t*>(args.layers)[e];
+    __syncthreads();
+    const MlpLayer* lay = L <= kSmemLayers ? s_lay : args.layers;
+    const int mt = (B + 15) / 16, mg = (mt + 1) / 2;  // blocks of 16 rows, taken in twos
+    Step st{args, lay, 0, make_float2(1.f, 1.f), 1.0, 1.0, mt};
+
+    // this CTA's shares of two task lists, dealt to its warps
+    auto for_tasks = [&](int n1, int n2, auto&& f1, auto&& f2) {
+        const int p1 = (n1 + nc - 1) / nc, p2 = (n2 + nc - 1) / nc;
+        const int s1 = min(n1, c * p1), e1 = min(n1, s1 + p1), s2 = min(n2, c * p2), e2 = min(n2, s2 + p2);
+        for (int k = warp; k < (e1 - s1) + (e2 - s2); k += kStepWarps) {
+            if (k < e1 - s1)
+                f1(s1 + k);
+            else
+                f2(s2 + k - (e1 - s1));
+        }
+        __syncwarp();
+    };
+    auto dw_tasks = [&](int l) { return (lay[l].doutp / 16) * (lay[l].dinp / 16) + (lay[l].dout + 31) / 32; };
+
+    // gather tasks of a step: operand blocks, then targets
+    const int kx = lay[0].dinp / 16, nx = mt * kx, nt = args.mode == kForward ? 0 : (B * args.out + 31) / 32;
+    auto gather = [&](int step, int task) {
+        if (task < nx)
+            gather_x(st, step, task / kx, task % kx);
+        else
+            gather_t(args, step, task - nx);
+    };
+    for_tasks(nx + nt, 0, [&](int task) { gather(0, task); }, [](int) {});
+    cluster_sync();
+
+    for (int step = 0; step < args.steps; step++) {
+        st.par = step & 1;
+        if (args.mode == kTrain) {
+            st.c12 = args.c12[step];
+            st.rc1 = 1.0 / (double)st.c12.x;
+            st.rc2 = 1.0 / (double)st.c12.y;
+        }
+
+        for (int l = 0; l < L; l++) {
+            for_tasks(mg * (lay[l].doutp / 8), 0, [&](int task) {
+                const int mb = 2 * (task % mg), nb = task / mg;
+                if (mb + 1 < mt)
+                    forward_tiles<2>(st, l, mb, nb);
+                else
+                    forward_tiles<1>(st, l, mb, nb);
+            }, [](int) {});
+            cluster_sync();
+        }
+        if (args.mode == kForward) continue;
+
+        // loss: mean over the batch of sum_o (y - t)^2 / out, by the last CTA
+        if (c == nc - 1) {
+            if (threadIdx.x < 256) {
+                float s = 0.f;
+                for (int i = threadIdx.x; i < B * args.out; i += 256) {
+                    const float df = args.yout[i] - st.tgt()[i];
+                    s += df * df;
+                }
+                red[threadIdx.x] = s;
+            }
+            __syncthreads();
+            for (int k = 128; k; k >>= 1) {
+                if (threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
+                __syncthreads();
+            }
+            if (threadIdx.x == 0) args.loss[step] = red[0] / (float)(B * args.out);
+        }
+        for (int l = L - 1; l >= 1; l--) {
+            for_tasks(mg * (lay[l].dinp / 8), l < L - 1 ? dw_tasks(l + 1) : 0, [&](int task) {
+                const int mb = 2 * (task % mg), nb = task / mg;
+                if (mb + 1 < mt)
+                    dx_tiles<2>(st, l, mb, nb);
+                else
+                    dx_tiles<1>(st, l, mb, nb);
+            }, [&](int task) { dw_task(st, l + 1, task); });
+            cluster_sync();
+        }
+        // the last phase also gathers the next step's rows
+        const int n0 = dw_tasks(0), ng = step + 1 < args.steps ? nx + nt : 0;
+        for_tasks(dw_tasks(1), n0 + ng, [&](int task) { dw_task(st, 1, task); }, [&](int task) {
+            if (task < ng)
+                gather(step + 1, task);
+            else
+                dw_task(st, 0, task - ng);
+        });
+        cluster_sync();
+    }
+}
+
+// Forward pass of 16 rows per CTA; the activations of two layers alternate in
+// shared memory as A blocks.  X and Y may be page-locked host memory.  Rows are
+// independent, so no CTA waits for another: 512 candidates on the 19-4x256-4
+// network are 32 CTAs that each read the 410 KB of BF16 weights from L2 (six
+// launches of a kernel per GEMM took 51-57 us each; 268 -> 64 us a call).
+__global__ void __launch_bounds__(kPredThreads) mlp_predict_kernel(const MlpLayer* layers, int L, int in, int out,
+                                                                   int n, int width, const float* bw, const float* X,
+                                                                   float* Y) {
+    extern __shared__ __align__(16) uint4 sact[];  // [2][width / 16][32]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int r0 = blockIdx.x * 16;
+    for (int k = warp; k < layers[0].dinp / 16; k += kPredWarps) {
+        auto pair = [&](int r, int c) {
+            const float* p = X + (size_t)r * in;
+            return r < n ? pack2(c < in ? p[c] : 0.f, c + 1 < in ? p[c + 1] : 0.f) : 0u;
+        };
+        const int c = 16 * k + 2 * t;
+        sact[32 * k + lane] =
+            make_uint4(pair(r0 + g, c), pair(r0 + g + 8, c), pair(r0 + g, c + 8), pair(r0 + g + 8, c + 8));
+    }
+    __syncthreads();
+    for (int l = 0; l < L; l++) {
+        const MlpLayer& y = layers[l];
+        const int kb = y.dinp / 16;
+        const uint4* src = sact + (l & 1) * 2 * width + lane;
+        uint4* dst = sact + ((l + 1) & 1) * 2 * width + lane;
+        for (int nb = warp; nb < y.doutp / 8; nb += kPredWarps) {
+            const uint2* wp = y.w + (size_t)nb * kb * 32 + lane;
+            const int c = 8 * nb + 2 * t;
+            const float2 bias = *reinterpret_cast<const float2*>(bw + y.bias + c);
+            float d[1][4];
+            mma_tiles<16, 1, 1>(kb, d, [&](int k, uint4 (&fa)[1], uint2 (&fb)[1]) {
+                fa[0] = src[32 * k];
+                fb[0] = wp[32 * k];
+            });
+            const float v[4] = {d[0][0] + bias.x, d[0][1] + bias.y, d[0][2] + bias.x, d[0][3] + bias.y};
+            if (l < L - 1) {
+                reinterpret_cast<uint2*>(dst + 32 * (nb / 2))[nb & 1] = make_uint2(
+                    pack2(fmaxf(v[0], 0.f), fmaxf(v[1], 0.f)), pack2(fmaxf(v[2], 0.f), fmaxf(v[3], 0.f)));
+                continue;
+            }
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const int m = m0 + wm + i * 16 + g + (q >= 2 ? 8 : 0);
-                const int n = n0 + wn + jn * 8 + 2 * t + (q & 1);
-                if (m >= op.M || n >= op.N) continue;
-                float v = op.alpha * acc[i][jn][q];
-                if (op.bias) v += op.bias[n];
-                if (op.relu) v = fmaxf(v, 0.f);
-                if (op.c_f32)
-                    static_cast<float*>(op.C)[m * op.ldc + n] = v;
-                else
-                    static_cast<__nv_bfloat16*>(op.C)[m * op.ldc + n] = __float2bfloat16_rn(v);
+                const int m = r0 + g + 8 * (q >> 1), o = c + (q & 1);
+                if (m < n && o < out) Y[(size_t)m * out + o] = v[q];
             }
-}
-
-// db[o] = sum_b dY[b][o] * (mask? Y[b][o] > 0)
-__global__ void bias_grad_kernel(const float* dY, const __nv_bfloat16* mask, int B, int O, float* db) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= O) return;
-    float s = 0.f;
-    for (int b = 0; b < B; b++) {
-        const float d = dY[(size_t)b * O + o];
-        if (!mask || __bfloat162float(mask[(size_t)b * O + o]) > 0.f) s += d;
-    }
-    db[o] = s;
-}
-
-// MSE over the batch: loss = mean_b sum_o (y - t)^2 / O; dY = 2 (y - t) / (B O)
-__global__ void mse_grad_kernel(const float* Y, const float* T, int B, int O, float* dY, float* loss) {
-    __shared__ float red[256];
-    float s = 0.f;
-    for (int i = threadIdx.x; i < B * O; i += blockDim.x) {
-        const float d = Y[i] - T[i];
-        dY[i] = 2.f * d / (float)(B * O);
-        s += d * d;
-    }
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+        }
         __syncthreads();
     }
-    if (threadIdx.x == 0) *loss = red[0] / (float)(B * O);
 }
 
-__global__ void adam_kernel(float* w, const float* g, float* m, float* v, __nv_bfloat16* w16, long long n, float lr,
-                            float b1, float b2, float eps, float c1, float c2) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.f - b1) * gi, vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-        w[i] = wi;
-        if (w16) w16[i] = __float2bfloat16_rn(wi);
+// One tile of a layer per warp, between the flat FP32 parameters and the
+// device's arrays: FP32 tiles and BF16 blocks from flat (pack), flat from the
+// tiles (unpack).  blockIdx.y: layer.
+__global__ void pack_kernel(const MlpLayer* layers, const float* flat, float4* w, float* bw) {
+    const MlpLayer& y = layers[blockIdx.y];
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, ot = y.doutp / 16, ki = y.dinp / 16;
+    const int warps = gridDim.x * (blockDim.x / 32), w0 = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    for (int k = w0; k < ot * (y.dinp / 8); k += warps) {
+        const int ob = k % ot, ib = k / ot;
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int o = 16 * ob + g + 8 * (q >> 1), i = 8 * ib + 2 * t + (q & 1);
+            v[q] = o < y.dout && i < y.din ? flat[y.woff + (long long)o * y.din + i] : 0.f;
+        }
+        w[(size_t)(y.tile + k) * 32 + lane] = make_float4(v[0], v[1], v[2], v[3]);
+        const uint32_t p0 = pack2(v[0], v[1]), p1 = pack2(v[2], v[3]);
+        uint32_t* wp = reinterpret_cast<uint32_t*>(y.w + ((size_t)(2 * ob) * ki + ib / 2) * 32 + lane) + (ib & 1);
+        wp[0] = p0;
+        wp[(size_t)ki * 64] = p1;
+        y.wt[((size_t)ib * ot + ob) * 32 + lane] = make_uint2(transpose8(p0), transpose8(p1));
     }
+    for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < y.doutp; o += gridDim.x * blockDim.x)
+        bw[y.bias + o] = o < y.dout ? flat[y.boff + o] : 0.f;
 }
 
-__global__ void to_bf16_kernel(const float* x, __nv_bfloat16* y, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        y[i] = __float2bfloat16_rn(x[i]);
-}
-
-__global__ void gather_rows_kernel(const float* X, const int* idx, int n, int d, float* out) {
-    const long long total = (long long)n * d;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-        const long long r = e / d, c = e % d;
-        out[e] = X[(long long)idx[r] * d + c];
+__global__ void unpack_kernel(const MlpLayer* layers, const float4* w, const float* bw, float* flat) {
+    const MlpLayer& y = layers[blockIdx.y];
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, ot = y.doutp / 16;
+    const int warps = gridDim.x * (blockDim.x / 32), w0 = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    for (int k = w0; k < ot * (y.dinp / 8); k += warps) {
+        const float4 f = w[(size_t)(y.tile + k) * 32 + lane];
+        const float v[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int o = 16 * (k % ot) + g + 8 * (q >> 1), i = 8 * (k / ot) + 2 * t + (q & 1);
+            if (o < y.dout && i < y.din) flat[y.woff + (long long)o * y.din + i] = v[q];
+        }
     }
+    for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < y.dout; o += gridDim.x * blockDim.x)
+        flat[y.boff + o] = bw[y.bias + o];
 }
 
-cudaError_t gemm(const GemmOp& op, cudaStream_t st) {
-    dim3 grid((op.N + TN - 1) / TN, (op.M + TM - 1) / TM);
-    gemm_bf16_kernel<<<grid, 128, 0, st>>>(op);
-    return cudaGetLastError();
-}
-
-GemmOp base_op() {
-    GemmOp o;
-    std::memset(&o, 0, sizeof o);
-    o.alpha = 1.f;
-    return o;
-}
+int pad16(int x) { return (x + 15) / 16 * 16; }
 
 }  // namespace
 
 struct bnm_mlp {
     int in = 0, hidden = 0, layers = 0, out = 0, max_batch = 0, device = 0;
     int L = 0;  // number of linear layers = layers + 1
-    std::vector<int> din, dout;
-    std::vector<long long> woff, boff;  // offsets into the flat parameter vector
+    std::vector<MlpLayer> lay;
+    MlpLayer* d_lay = nullptr;
     long long n_params = 0;
+    int cluster = 8;        // CTAs of mlp_step_kernel
+    int width = 0;          // widest padded layer input
+    size_t pred_smem = 0;   // shared memory of mlp_predict_kernel, 0: too wide for it
+    int pred_rows = 0;      // rows per predict launch
     cudaStream_t st = nullptr;
-    float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;  // flat [W_l (out x in), b_l (out)]...
-    __nv_bfloat16* w16 = nullptr;
-    std::vector<__nv_bfloat16*> act;  // act[0] = input (bf16), act[l] = hidden outputs (bf16)
-    float* yout = nullptr;            // [max_batch][out] last-layer output (f32)
-    float *dA = nullptr, *dB = nullptr;  // gradient ping-pong [max_batch][max width]
-    float* loss = nullptr;
-    float *xin = nullptr, *tgt = nullptr;  // staged batch input / target (f32)
+    long long n_tiles = 0, n_bias = 0;
+    float4 *w = nullptr, *m = nullptr, *v = nullptr;     // weights and Adam moments, [tile][lane]
+    float *bw = nullptr, *bm = nullptr, *bv = nullptr;   // biases and theirs
+    float* flat = nullptr;  // parameters or gradient in the caller's order: [W_l (out x in), b_l (out)]...
+    float* yout = nullptr;  // [max_batch][out] last-layer output (f32)
+    float* loss = nullptr;  // [kMaxSteps]
+    float2* c12 = nullptr;  // [kMaxSteps]
+    float *xin = nullptr, *tgt = nullptr;        // staged batch input / target (f32)
+    float* tgt2 = nullptr;  // targets of the rows of two steps
+    float *io = nullptr;                         // page-locked rows in and out of predict
     float *data_x = nullptr, *data_y = nullptr;  // training set on the device
-    int* idx = nullptr;
     long long data_n = 0;
+    int* idx = nullptr;  // row indices of the steps of one launch
+    size_t idx_cap = 0;
     int adam_t = 0;
-    std::vector<void*> allocs;
+    void* slab = nullptr;  // the device buffers above, except the growing ones (data_x, data_y, idx)
 };
 
-static int mlp_alloc(bnm_mlp* p, void** ptr, size_t bytes) {
-    cudaError_t e = cudaMalloc(ptr, bytes ? bytes : 16);
-    if (e != cudaSuccess) return bnm_fail_cuda(e, "cudaMalloc", __FILE__, __LINE__);
-    p->allocs.push_back(*ptr);
-    return BNM_OK;
-}
+// Training steps per launch: bounds the index buffer and the time one launch holds its SMs.
+static constexpr int kMaxSteps = 2048;
 
 extern "C" void bnm_mlp_destroy(bnm_mlp* p) {
     if (!p) return;
     cudaSetDevice(p->device);
     if (p->st) cudaStreamSynchronize(p->st);
-    for (void* a : p->allocs) cudaFree(a);
+    for (void* a : {p->slab, (void*)p->data_x, (void*)p->data_y, (void*)p->idx})
+        if (a) cudaFree(a);
+    if (p->io) cudaFreeHost(p->io);
     if (p->st) cudaStreamDestroy(p->st);
     delete p;
+}
+
+// Device arrays from the flat parameters, Adam's state cleared (asynchronous)
+static cudaError_t load_flat(bnm_mlp* p) {
+    pack_kernel<<<dim3(64, p->L), 256, 0, p->st>>>(p->d_lay, p->flat, p->w, p->bw);
+    cudaError_t e = cudaGetLastError();
+    // m, v, bm, bv follow one another in the slab
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(p->m, 0, (size_t)((char*)(p->bv + p->n_bias) - (char*)p->m), p->st);
+    return e;
+}
+
+static int mlp_init(bnm_mlp* p, uint64_t seed) {
+    BNM_CUDA_TRY(cudaSetDevice(p->device));
+    BNM_CUDA_TRY(cudaStreamCreateWithFlags(&p->st, cudaStreamNonBlocking));
+    const size_t np = (size_t)p->n_params, rows = pad16(p->max_batch);
+    const size_t tb = (size_t)p->n_tiles * 32 * sizeof(float4), bb = (size_t)p->n_bias * 4;
+    // every buffer is a piece of one allocation: sized first, then placed
+    for (int pass = 0; pass < 2; pass++) {
+        unsigned char* base = pass ? static_cast<unsigned char*>(p->slab) : nullptr;
+        size_t off = 0;
+        auto take = [&](auto*& field, size_t bytes) {
+            if (pass) field = reinterpret_cast<std::remove_reference_t<decltype(field)>>(base + off);
+            off += (bytes + 255) / 256 * 256;
+        };
+        take(p->m, tb);
+        take(p->v, tb);
+        take(p->bm, bb);
+        take(p->bv, bb);
+        take(p->w, tb);
+        take(p->bw, bb);
+        take(p->flat, np * 4);
+        for (MlpLayer& y : p->lay) {
+            take(y.w, (size_t)y.dinp * y.doutp * 2);
+            take(y.wt, (size_t)y.dinp * y.doutp * 2);
+            p->width = std::max(p->width, y.dinp);
+        }
+        take(p->yout, (size_t)p->max_batch * p->out * 4);
+        take(p->loss, (size_t)kMaxSteps * 4);
+        take(p->c12, (size_t)kMaxSteps * 8);
+        take(p->xin, (size_t)p->max_batch * p->in * 4);
+        take(p->tgt, (size_t)p->max_batch * p->out * 4);
+        take(p->tgt2, (size_t)2 * p->max_batch * p->out * 4);
+        for (MlpLayer& y : p->lay) {
+            const size_t sets = &y == &p->lay[0] ? 2 : 1;
+            take(y.x, sets * rows * y.dinp * 2);
+            take(y.xt, sets * rows * y.dinp * 2);
+            take(y.dz, (size_t)p->max_batch * y.doutp * 4);
+            take(y.dzh, rows * y.doutp * 2);
+            take(y.dzt, rows * y.doutp * 2);
+        }
+        take(p->d_lay, p->lay.size() * sizeof(MlpLayer));
+        if (!pass) BNM_CUDA_TRY(cudaMalloc(&p->slab, off));
+    }
+    BNM_CUDA_TRY(cudaMemcpyAsync(p->d_lay, p->lay.data(), p->lay.size() * sizeof(MlpLayer), cudaMemcpyHostToDevice,
+                                 p->st));
+    // predict: rows travel through a page-locked buffer of at most 16 MiB (or max_batch rows)
+    const size_t row_bytes = (size_t)(p->in + p->out) * 4;
+    p->pred_rows = (int)std::max<size_t>(p->max_batch, std::min<size_t>(8192, ((size_t)16 << 20) / row_bytes));
+    p->pred_smem = (size_t)2 * 16 * p->width * 2;
+    if (p->pred_smem > 200 * 1024) p->pred_smem = 0;
+    if (p->pred_smem) {
+        BNM_CUDA_TRY(cudaFuncSetAttribute(mlp_predict_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)p->pred_smem));
+    }
+    // 16 CTAs where the GPU can place such a cluster, else the portable 8
+    BNM_CUDA_TRY(cudaFuncSetAttribute(mlp_step_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof cfg);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 16;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(kStepThreads);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, mlp_step_kernel, &cfg) == cudaSuccess && clusters > 0)
+        p->cluster = 16;
+    cudaGetLastError();
+    // He-uniform initialisation (host, seeded), zero biases; Adam state zero
+    std::vector<float> w0(np, 0.f);
+    std::mt19937_64 gen(seed);
+    for (const MlpLayer& y : p->lay) {
+        const float lim = std::sqrt(6.0f / (float)y.din);
+        std::uniform_real_distribution<float> U(-lim, lim);
+        for (long long i = 0; i < (long long)y.din * y.dout; i++) w0[y.woff + i] = U(gen);
+    }
+    BNM_CUDA_TRY(cudaMemcpyAsync(p->flat, w0.data(), np * 4, cudaMemcpyHostToDevice, p->st));
+    BNM_CUDA_TRY(load_flat(p));
+    BNM_CUDA_TRY(cudaStreamSynchronize(p->st));
+    return BNM_OK;
 }
 
 extern "C" int bnm_mlp_create(int32_t in_dim, int32_t hidden, int32_t layers, int32_t out_dim, int32_t max_batch,
@@ -258,68 +783,24 @@ extern "C" int bnm_mlp_create(int32_t in_dim, int32_t hidden, int32_t layers, in
     p->device = device;
     p->L = layers + 1;
     for (int l = 0; l < p->L; l++) {
-        p->din.push_back(l == 0 ? in_dim : hidden);
-        p->dout.push_back(l == p->L - 1 ? out_dim : hidden);
-        p->woff.push_back(p->n_params);
-        p->n_params += (long long)p->din[l] * p->dout[l];
-        p->boff.push_back(p->n_params);
-        p->n_params += p->dout[l];
+        MlpLayer y;
+        std::memset(&y, 0, sizeof y);
+        y.din = l == 0 ? in_dim : hidden;
+        y.dout = l == p->L - 1 ? out_dim : hidden;
+        y.dinp = pad16(y.din);
+        y.doutp = pad16(y.dout);
+        y.woff = p->n_params;
+        p->n_params += (long long)y.din * y.dout;
+        y.boff = p->n_params;
+        p->n_params += y.dout;
+        y.tile = p->n_tiles;
+        p->n_tiles += (long long)(y.doutp / 16) * (y.dinp / 8);
+        y.bias = p->n_bias;
+        p->n_bias += y.doutp;
+        p->lay.push_back(y);
     }
-    int rc = BNM_OK;
-    cudaError_t e = cudaSetDevice(device);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->st, cudaStreamNonBlocking);
-    if (e != cudaSuccess) {
-        rc = bnm_fail_cuda(e, "cudaSetDevice/cudaStreamCreate", __FILE__, __LINE__);
-        bnm_mlp_destroy(p);
-        return rc;
-    }
-    const size_t np = (size_t)p->n_params;
-    const int wmax = std::max(std::max(in_dim, hidden), out_dim);
-    void* ptr;
-#define MLP_ALLOC(field, bytes)                                   \
-    if ((rc = mlp_alloc(p, &ptr, (bytes)))) {                     \
-        bnm_mlp_destroy(p);                                       \
-        return rc;                                                \
-    }                                                             \
-    p->field = static_cast<decltype(p->field)>(ptr);
-    MLP_ALLOC(w, np * 4);
-    MLP_ALLOC(g, np * 4);
-    MLP_ALLOC(m, np * 4);
-    MLP_ALLOC(v, np * 4);
-    MLP_ALLOC(w16, np * 2);
-    MLP_ALLOC(yout, (size_t)max_batch * out_dim * 4);
-    MLP_ALLOC(dA, (size_t)max_batch * wmax * 4);
-    MLP_ALLOC(dB, (size_t)max_batch * wmax * 4);
-    MLP_ALLOC(loss, 16);
-    MLP_ALLOC(xin, (size_t)max_batch * in_dim * 4);
-    MLP_ALLOC(tgt, (size_t)max_batch * out_dim * 4);
-    MLP_ALLOC(idx, (size_t)max_batch * 4);
-#undef MLP_ALLOC
-    p->act.assign(p->L, nullptr);
-    for (int l = 0; l < p->L; l++) {
-        if ((rc = mlp_alloc(p, &ptr, (size_t)max_batch * p->din[l] * 2))) {
-            bnm_mlp_destroy(p);
-            return rc;
-        }
-        p->act[l] = static_cast<__nv_bfloat16*>(ptr);
-    }
-    // He-uniform initialisation (host, seeded), zero biases; Adam state zero
-    std::vector<float> w0(np, 0.f);
-    std::mt19937_64 gen(seed);
-    for (int l = 0; l < p->L; l++) {
-        const float lim = std::sqrt(6.0f / (float)p->din[l]);
-        std::uniform_real_distribution<float> U(-lim, lim);
-        for (long long i = 0; i < (long long)p->din[l] * p->dout[l]; i++) w0[p->woff[l] + i] = U(gen);
-    }
-    e = cudaMemcpy(p->w, w0.data(), np * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(p->m, 0, np * 4);
-    if (e == cudaSuccess) e = cudaMemset(p->v, 0, np * 4);
-    if (e == cudaSuccess) {
-        to_bf16_kernel<<<256, 256, 0, p->st>>>(p->w, p->w16, (long long)np);
-        e = cudaStreamSynchronize(p->st);
-    }
-    if (e != cudaSuccess) {
-        rc = bnm_fail_cuda(e, "MLP initialisation", __FILE__, __LINE__);
+    const int rc = mlp_init(p, seed);
+    if (rc) {
         bnm_mlp_destroy(p);
         return rc;
     }
@@ -327,92 +808,71 @@ extern "C" int bnm_mlp_create(int32_t in_dim, int32_t hidden, int32_t layers, in
     return BNM_OK;
 }
 
-// forward pass of a staged batch (xin f32 [B][in]) into yout
-static int forward(bnm_mlp* p, int B) {
-    to_bf16_kernel<<<64, 256, 0, p->st>>>(p->xin, p->act[0], (long long)B * p->in);
-    for (int l = 0; l < p->L; l++) {
-        GemmOp o = base_op();
-        o.M = B;
-        o.N = p->dout[l];
-        o.K = p->din[l];
-        o.A = p->act[l];
-        o.sam = p->din[l];
-        o.sak = 1;
-        o.B = p->w16 + p->woff[l];  // W_l [out][in]: B(k=in, n=out) = W[n*in + k]
-        o.sbk = 1;
-        o.sbn = p->din[l];
-        o.bias = p->w + p->boff[l];
-        const bool last = l == p->L - 1;
-        o.relu = !last;
-        o.C = last ? (void*)p->yout : (void*)p->act[l + 1];
-        o.ldc = p->dout[l];
-        o.c_f32 = last;
-        BNM_CUDA_TRY(gemm(o, p->st));
-    }
-    return BNM_OK;
+static StepArgs step_args(bnm_mlp* p, int mode, int batch, const float* X, const float* T) {
+    StepArgs a;
+    std::memset(&a, 0, sizeof a);
+    a.layers = p->d_lay;
+    a.L = p->L;
+    a.in = p->in;
+    a.out = p->out;
+    a.mode = mode;
+    a.steps = 1;
+    a.batch = batch;
+    a.w = p->w;
+    a.m = p->m;
+    a.v = p->v;
+    a.bw = p->bw;
+    a.bm = p->bm;
+    a.bv = p->bv;
+    a.g = p->flat;
+    a.X = X;
+    a.T = T;
+    a.c12 = p->c12;
+    a.x0 = (size_t)pad16(p->max_batch) * p->lay[0].dinp * 2 / sizeof(uint4);
+    a.xt0 = 2 * a.x0;
+    a.tgt = p->tgt2;
+    a.yout = p->yout;
+    a.loss = p->loss;
+    return a;
 }
 
-// loss and gradients of the staged batch (xin, tgt) into p->g
-static int backward(bnm_mlp* p, int B) {
-    mse_grad_kernel<<<1, 256, 0, p->st>>>(p->yout, p->tgt, B, p->out, p->dA, p->loss);
-    float* dY = p->dA;
-    float* dX = p->dB;
-    for (int l = p->L - 1; l >= 0; l--) {
-        const bool last = l == p->L - 1;
-        // the ReLU of layer l's output (hidden layers) masks dY
-        const __nv_bfloat16* mask = last ? nullptr : p->act[l + 1];
-        bias_grad_kernel<<<(p->dout[l] + 127) / 128, 128, 0, p->st>>>(dY, mask, B, p->dout[l], p->g + p->boff[l]);
-        // dW[o][i] = sum_b dZ[b][o] X[b][i]
-        GemmOp gw = base_op();
-        gw.M = p->dout[l];
-        gw.N = p->din[l];
-        gw.K = B;
-        gw.A = dY;
-        gw.a_f32 = 1;
-        gw.sam = 1;
-        gw.sak = p->dout[l];
-        gw.mask = mask;
-        gw.smm = 1;
-        gw.smk = p->dout[l];
-        gw.B = p->act[l];
-        gw.sbk = p->din[l];
-        gw.sbn = 1;
-        gw.C = p->g + p->woff[l];
-        gw.ldc = p->din[l];
-        gw.c_f32 = 1;
-        BNM_CUDA_TRY(gemm(gw, p->st));
-        if (l == 0) break;
-        // dX[b][i] = sum_o dZ[b][o] W[o][i]
-        GemmOp gx = base_op();
-        gx.M = B;
-        gx.N = p->din[l];
-        gx.K = p->dout[l];
-        gx.A = dY;
-        gx.a_f32 = 1;
-        gx.sam = p->dout[l];
-        gx.sak = 1;
-        gx.mask = mask;
-        gx.smm = p->dout[l];
-        gx.smk = 1;
-        gx.B = p->w16 + p->woff[l];
-        gx.sbk = p->din[l];
-        gx.sbn = 1;
-        gx.C = dX;
-        gx.ldc = p->din[l];
-        gx.c_f32 = 1;
-        BNM_CUDA_TRY(gemm(gx, p->st));
-        std::swap(dY, dX);
-    }
+static int launch_step(bnm_mlp* p, const StepArgs& a) {
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof cfg);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p->cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)p->cluster);
+    cfg.blockDim = dim3(kStepThreads);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.stream = p->st;
+    BNM_CUDA_TRY(cudaLaunchKernelEx(&cfg, mlp_step_kernel, a));
     return BNM_OK;
 }
 
 extern "C" int bnm_mlp_predict(bnm_mlp* p, const float* X, int32_t n, float* Y) {
     if (!p || !X || !Y || n < 0) return bnm_fail_msg(BNM_EINVAL, "bad predict arguments");
     BNM_CUDA_TRY(cudaSetDevice(p->device));
+    if (p->pred_smem) {
+        if (!p->io) BNM_CUDA_TRY(cudaMallocHost((void**)&p->io, (size_t)p->pred_rows * (p->in + p->out) * 4));
+        float* io_y = p->io + (size_t)p->pred_rows * p->in;
+        for (int s = 0; s < n; s += p->pred_rows) {
+            const int B = std::min(p->pred_rows, n - s);
+            std::memcpy(p->io, X + (size_t)s * p->in, (size_t)B * p->in * 4);
+            mlp_predict_kernel<<<(B + 15) / 16, kPredThreads, p->pred_smem, p->st>>>(p->d_lay, p->L, p->in, p->out, B,
+                                                                                   p->width, p->bw, p->io, io_y);
+            BNM_CUDA_TRY(cudaGetLastError());
+            BNM_CUDA_TRY(cudaStreamSynchronize(p->st));
+            std::memcpy(Y + (size_t)s * p->out, io_y, (size_t)B * p->out * 4);
+        }
+        return BNM_OK;
+    }
     for (int s = 0; s < n; s += p->max_batch) {
         const int B = std::min(p->max_batch, n - s);
         BNM_CUDA_TRY(cudaMemcpyAsync(p->xin, X + (size_t)s * p->in, (size_t)B * p->in * 4, cudaMemcpyHostToDevice, p->st));
-        int rc = forward(p, B);
+        int rc = launch_step(p, step_args(p, kForward, B, p->xin, nullptr));
         if (rc) return rc;
         BNM_CUDA_TRY(cudaMemcpyAsync(Y + (size_t)s * p->out, p->yout, (size_t)B * p->out * 4, cudaMemcpyDeviceToHost, p->st));
     }
@@ -426,11 +886,10 @@ extern "C" int bnm_mlp_loss_and_grads(bnm_mlp* p, const float* X, const float* T
     BNM_CUDA_TRY(cudaSetDevice(p->device));
     BNM_CUDA_TRY(cudaMemcpyAsync(p->xin, X, (size_t)n * p->in * 4, cudaMemcpyHostToDevice, p->st));
     BNM_CUDA_TRY(cudaMemcpyAsync(p->tgt, T, (size_t)n * p->out * 4, cudaMemcpyHostToDevice, p->st));
-    int rc = forward(p, n);
-    if (!rc) rc = backward(p, n);
+    int rc = launch_step(p, step_args(p, kGrads, n, p->xin, p->tgt));
     if (rc) return rc;
     if (loss) BNM_CUDA_TRY(cudaMemcpyAsync(loss, p->loss, 4, cudaMemcpyDeviceToHost, p->st));
-    if (grads) BNM_CUDA_TRY(cudaMemcpyAsync(grads, p->g, (size_t)p->n_params * 4, cudaMemcpyDeviceToHost, p->st));
+    if (grads) BNM_CUDA_TRY(cudaMemcpyAsync(grads, p->flat, (size_t)p->n_params * 4, cudaMemcpyDeviceToHost, p->st));
     BNM_CUDA_TRY(cudaStreamSynchronize(p->st));
     return BNM_OK;
 }
@@ -440,47 +899,74 @@ extern "C" int bnm_mlp_train(bnm_mlp* p, const float* X, const float* Y, int32_t
     if (!p || !X || !Y || n < 1 || batch < 1 || batch > p->max_batch || epochs < 0)
         return bnm_fail_msg(BNM_EINVAL, "bad training arguments");
     BNM_CUDA_TRY(cudaSetDevice(p->device));
+    const int nb = n / batch;  // full batches only
     if (p->data_n < n) {
-        if (p->data_x) {
-            cudaFree(p->data_x);
-            cudaFree(p->data_y);
+        for (float** q : {&p->data_x, &p->data_y}) {
+            if (*q) cudaFree(*q);
+            *q = nullptr;
         }
+        p->data_n = 0;
         BNM_CUDA_TRY(cudaMalloc(&p->data_x, (size_t)n * p->in * 4));
         BNM_CUDA_TRY(cudaMalloc(&p->data_y, (size_t)n * p->out * 4));
         p->data_n = n;
-        p->allocs.push_back(p->data_x);
-        p->allocs.push_back(p->data_y);
+    }
+    const long long total = (long long)nb * epochs;
+    const size_t need = (size_t)std::min<long long>(total, kMaxSteps) * batch;
+    if (p->idx_cap < need) {
+        if (p->idx) cudaFree(p->idx);
+        p->idx = nullptr;
+        p->idx_cap = 0;
+        BNM_CUDA_TRY(cudaMalloc(&p->idx, need * 4));
+        p->idx_cap = need;
     }
     BNM_CUDA_TRY(cudaMemcpyAsync(p->data_x, X, (size_t)n * p->in * 4, cudaMemcpyHostToDevice, p->st));
     BNM_CUDA_TRY(cudaMemcpyAsync(p->data_y, Y, (size_t)n * p->out * 4, cudaMemcpyHostToDevice, p->st));
-    std::vector<int> order(n);
+    std::vector<int> order(n), idx;
     for (int i = 0; i < n; i++) order[i] = i;
     std::mt19937_64 gen(shuffle_seed);
-    std::vector<float> losses;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    std::vector<float2> c12;
+    std::vector<float> losses((size_t)total);
+    long long done = 0;
+    // one launch per kMaxSteps steps
+    auto flush = [&]() -> int {
+        const int steps = (int)c12.size();
+        if (!steps) return BNM_OK;
+        BNM_CUDA_TRY(cudaMemcpyAsync(p->idx, idx.data(), idx.size() * 4, cudaMemcpyHostToDevice, p->st));
+        BNM_CUDA_TRY(cudaMemcpyAsync(p->c12, c12.data(), (size_t)steps * 8, cudaMemcpyHostToDevice, p->st));
+        StepArgs a = step_args(p, kTrain, batch, p->data_x, p->data_y);
+        a.steps = steps;
+        a.idx = p->idx;
+        a.lr = lr;
+        a.b1 = b1;
+        a.b2 = b2;
+        a.eps = eps;
+        int rc = launch_step(p, a);
+        if (rc) return rc;
+        BNM_CUDA_TRY(cudaMemcpyAsync(losses.data() + done, p->loss, (size_t)steps * 4, cudaMemcpyDeviceToHost, p->st));
+        BNM_CUDA_TRY(cudaStreamSynchronize(p->st));
+        done += steps;
+        idx.clear();
+        c12.clear();
+        return BNM_OK;
+    };
+    int rc;
     for (int ep = 0; ep < epochs; ep++) {
         std::shuffle(order.begin(), order.end(), gen);
-        double sum = 0.0;
-        int nb = 0;
-        for (int s = 0; s + batch <= n; s += batch) {  // full batches only
-            BNM_CUDA_TRY(cudaMemcpyAsync(p->idx, order.data() + s, (size_t)batch * 4, cudaMemcpyHostToDevice, p->st));
-            gather_rows_kernel<<<64, 256, 0, p->st>>>(p->data_x, p->idx, batch, p->in, p->xin);
-            gather_rows_kernel<<<64, 256, 0, p->st>>>(p->data_y, p->idx, batch, p->out, p->tgt);
-            int rc = forward(p, batch);
-            if (!rc) rc = backward(p, batch);
-            if (rc) return rc;
+        for (int s = 0; s < nb; s++) {
+            idx.insert(idx.end(), order.begin() + (size_t)s * batch, order.begin() + (size_t)(s + 1) * batch);
             p->adam_t++;
-            const float c1 = 1.f - std::pow(b1, (float)p->adam_t), c2 = 1.f - std::pow(b2, (float)p->adam_t);
-            adam_kernel<<<256, 256, 0, p->st>>>(p->w, p->g, p->m, p->v, p->w16, p->n_params, lr, b1, b2, eps, c1, c2);
-            float l = 0.f;
-            BNM_CUDA_TRY(cudaMemcpyAsync(&l, p->loss, 4, cudaMemcpyDeviceToHost, p->st));
-            BNM_CUDA_TRY(cudaStreamSynchronize(p->st));  // the index buffer is reused next batch
-            sum += l;
-            nb++;
+            c12.push_back(make_float2(1.f - std::pow(b1, (float)p->adam_t), 1.f - std::pow(b2, (float)p->adam_t)));
+            if ((int)c12.size() == kMaxSteps && (rc = flush())) return rc;
         }
-        if (loss_per_epoch) loss_per_epoch[ep] = nb ? (float)(sum / nb) : 0.f;
     }
-    BNM_CUDA_TRY(cudaGetLastError());
+    if ((rc = flush())) return rc;
+    BNM_CUDA_TRY(cudaStreamSynchronize(p->st));
+    for (int ep = 0; loss_per_epoch && ep < epochs; ep++) {
+        double sum = 0.0;
+        for (int s = 0; s < nb; s++) sum += losses[(size_t)ep * nb + s];
+        loss_per_epoch[ep] = nb ? (float)(sum / nb) : 0.f;
+    }
     return BNM_OK;
 }
 
@@ -489,19 +975,20 @@ extern "C" int64_t bnm_mlp_num_params(const bnm_mlp* p) { return p ? p->n_params
 extern "C" int bnm_mlp_get_params(bnm_mlp* p, float* flat) {
     if (!p || !flat) return bnm_fail_msg(BNM_EINVAL, "null argument");
     BNM_CUDA_TRY(cudaSetDevice(p->device));
-    BNM_CUDA_TRY(cudaMemcpy(flat, p->w, (size_t)p->n_params * 4, cudaMemcpyDeviceToHost));
+    unpack_kernel<<<dim3(64, p->L), 256, 0, p->st>>>(p->d_lay, p->w, p->bw, p->flat);
+    BNM_CUDA_TRY(cudaGetLastError());
+    BNM_CUDA_TRY(cudaMemcpyAsync(flat, p->flat, (size_t)p->n_params * 4, cudaMemcpyDeviceToHost, p->st));
+    BNM_CUDA_TRY(cudaStreamSynchronize(p->st));
     return BNM_OK;
 }
 
 extern "C" int bnm_mlp_set_params(bnm_mlp* p, const float* flat) {
     if (!p || !flat) return bnm_fail_msg(BNM_EINVAL, "null argument");
     BNM_CUDA_TRY(cudaSetDevice(p->device));
-    BNM_CUDA_TRY(cudaMemcpy(p->w, flat, (size_t)p->n_params * 4, cudaMemcpyHostToDevice));
+    BNM_CUDA_TRY(cudaMemcpyAsync(p->flat, flat, (size_t)p->n_params * 4, cudaMemcpyHostToDevice, p->st));
     // new parameters start a new optimisation: Adam's moments and step count restart
-    BNM_CUDA_TRY(cudaMemsetAsync(p->m, 0, (size_t)p->n_params * 4, p->st));
-    BNM_CUDA_TRY(cudaMemsetAsync(p->v, 0, (size_t)p->n_params * 4, p->st));
     p->adam_t = 0;
-    to_bf16_kernel<<<256, 256, 0, p->st>>>(p->w, p->w16, p->n_params);
+    BNM_CUDA_TRY(load_flat(p));
     BNM_CUDA_TRY(cudaStreamSynchronize(p->st));
     return BNM_OK;
 }
