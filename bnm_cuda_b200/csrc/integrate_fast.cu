@@ -604,18 +604,7 @@ cudaError_t bnm_launch_integrate_shape(const bnm::SimArgs& a, const bnm::Integra
         return bnm_launch_integrate_colsplit(b, sh.csize, sh.rpw, sh.slots, sh.kr, sh.kind == 4 ? 2 : 1, st);
     }
     if (sh.kind != 2 || !a.noise) return cudaErrorInvalidValue;  // the reference-order kernel reads a table
-    const int threads = ((a.N + 31) / 32) * 32;
-    if (threads > 1024) return cudaErrorInvalidValue;
-    size_t smem = 2 * (size_t)threads * sizeof(float);
-    const size_t sc_bytes = (size_t)a.N * a.sc_ld * sizeof(float);
-    int sc_in_smem = (smem + sc_bytes) <= 200 * 1024;
-    if (sc_in_smem) smem += sc_bytes;
-    cudaError_t e = cudaFuncSetAttribute(fastgen::integrate_generic_kernel<float>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    const int grid = a.n_sims < 2 * num_sms ? a.n_sims : 2 * num_sms;
-    fastgen::integrate_generic_kernel<float><<<grid, threads, smem, st>>>(a, sc_in_smem);
-    return cudaGetLastError();
+    return fastgen::launch_generic<float>(a, num_sms, st);
 }
 
 double bnm_integrator_share(const bnm::SimArgs& a, const bnm::IntegratorShape& sh, int num_sms) {
