@@ -11,11 +11,11 @@
 //   FIC penalty bnm.cpp:389-405, bnm.cu:752-767
 //
 // B200 layout:
-//   * fc_window_kernel: one CTA per (simulation, chunk of pairs).  BOLD frames
-//     stream through a shared-memory ring; every pair keeps FP64 running
-//     co-moments of the globally centred series, updated by one add and one
-//     subtract per frame as the window slides, so window FC costs O(P) per
-//     window instead of O(P*L).  Static FC comes from the same pass.  Window
+//   * fc_window_kernel: one CTA per (tile of node pairs, simulation).  BOLD
+//     frames stream through a shared-memory ring as centred FP64 values; every
+//     pair keeps FP64 running co-moments, updated by one add and one subtract
+//     per frame as the window slides, so window FC costs O(P) per window
+//     instead of O(P*L).  Static FC comes from the same pass.  Window
 //     sums over pairs (for the FCD centring) follow in window_sums_kernel,
 //     FP64 in a fixed order, so the FCD does not depend on the window tile.
 //   * fcd_gram_kernel: FCD = Z Z^T over the centred, unit-norm window-FC rows
@@ -24,6 +24,7 @@
 //     empirical FCD), so FCD never has to be sorted.
 //   * gof_kernel: prefix-scan of that histogram gives the exact KS statistic;
 //     FC correlation / mean difference in FP64; cost assembly.
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "kernels.h"
@@ -37,118 +38,279 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-template <typename TB, int PPT>
-__global__ void __launch_bounds__(256) fc_window_kernel(FcArgs a, const TB* __restrict__ bold) {
+// ------------------------------------------------------------ window FC
+//
+// Threads: 256 that own RI x RJ pairs each (thread (ty, tx): nodes i0 + ty +
+// 16 a and j0 + tx + 16 b), and one per node of the tile (its 16 RI rows and
+// 16 RJ columns) that centres the node's series, writes it to the ring and
+// keeps the node's window sums, a chunk of kChunk frames ahead of the pairs.
+//
+// What bounds it: the FP64 pipe, about 15 operations a pair and window (three
+// co-moment updates, the covariance, and the quotient below), at 16 lanes per
+// cycle of an SM quarter.  The former kernel took pairs from a table: each
+// read four series values and converted and centred them itself, every frame
+// cost two block barriers, and the quotient was CUDA's square root and
+// division, a branch each: 7.6 ms at N = 400, 4 series of 1201 frames (79,800
+// pairs, 1157 windows; now 1.3 ms), 1.35 ms at N = 100, 64 series of 585
+// frames (now 0.63 ms).
+constexpr int kChunk = 8;
+
+// (float)(cov / sqrt(vi vj)) as the plain FP64 expression gives it.
+__device__ __noinline__ double corr_plain(double cov, double vi, double vj) { return cov / sqrt(vi * vj); }
+// The same FP32 value without the branches of the division and square root:
+// the product with a reciprocal root from two Newton steps is within 2^-50 of
+// the plain expression, so both round to the same FP32 value unless that
+// interval holds the midpoint of two FP32 neighbours, or the value is below
+// FP32's normal range; those have to be done over (redo).  vi and vj inside
+// var_ok's range.
+__device__ __forceinline__ double corr_fast(double cov, double vi, double vj, bool& redo) {
+    const double p = vi * vj, h = 0.5 * p;
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(p));
+    y = fma(y, fma(-h, y * y, 0.5), y);
+    y = fma(y, fma(-h, y * y, 0.5), y);
+    const double r = cov * y;
+    const unsigned lo = ((unsigned)__double2loint(r) - (0x10000000u - 128u)) & 0x1fffffffu;  // bits below FP32's last
+    redo = lo <= 256u || ((unsigned)__double2hiint(r) & 0x7fffffffu) < 0x38200000u;            // |r| < 2^-125
+    return r;
+}
+// 2^-450 <= v < 2^450: products and their reciprocal roots keep full precision
+__device__ __forceinline__ bool var_ok(double v) {
+    return (unsigned)__double2hiint(v) - 0x23d00000u < 0x5c100000u - 0x23d00000u;
+}
+
+// Shared memory: ring [rl][NT] double, window sums [2][kChunk][NT] double2
+// (sum, variance sum), node means [NT], series sums [NT] double2, and per
+// window slot whether a variance was outside var_ok's range (int [2][kChunk + 1],
+// the last for the series).
+template <typename TB, int RI, int RJ, bool kRing>
+__global__ void __launch_bounds__(256 + (RI + RJ + 1) / 2 * 32) fc_window_kernel(FcArgs a, const TB* __restrict__ bold,
+                                                                                 int rl) {
+    constexpr int TI = 16 * RI, TJ = 16 * RJ, NT = TI + TJ;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int N = a.N, L = a.win_len;
-    double* mean = reinterpret_cast<double*>(smem_raw);  // [N]
-    double* fs = mean + N;                                // full-series sums [N]
-    double* fss = fs + N;
-    double* ws = fss + N;                                 // current-window sums [N]
-    double* wss = ws + N;
-    TB* ring = reinterpret_cast<TB*>(wss + N);            // last L frames [L][N]
-
-    const int sim = blockIdx.x;
-    const int p0 = blockIdx.y * (blockDim.x * PPT);
-    const size_t base = ((size_t)sim * a.frames + a.n_vols_remove) * N;
-    const int T0 = a.corr_len;
-
-    // node means over the kept frames (FP64); the series are centred on them
-    for (int n = threadIdx.x; n < N; n += blockDim.x) {
-        double s = 0.0;
-        for (int t = 0; t < T0; t++) s += (double)bold[base + (size_t)t * N + n];
-        mean[n] = s / T0;
-        fs[n] = fss[n] = ws[n] = wss[n] = 0.0;
-    }
-    int pi[PPT], pj[PPT];
-    bool pv[PPT];
-    double full[PPT], win[PPT];
-#pragma unroll
-    for (int u = 0; u < PPT; u++) {
-        const int p = p0 + u * blockDim.x + threadIdx.x;
-        pv[u] = p < a.P;
-        pi[u] = pv[u] ? a.pair_i[p] : 0;
-        pj[u] = pv[u] ? a.pair_j[p] : 0;
-        full[u] = win[u] = 0.0;
-    }
-    int k = 0, lo = 0;  // current window and the first frame it covers
-    bool any_nan = false;
+    double* ring = reinterpret_cast<double*>(smem_raw);
+    double2* stat = reinterpret_cast<double2*>(ring + (size_t)rl * NT);
+    double2* series = stat + 2 * kChunk * NT;
+    double* mean = reinterpret_cast<double*>(series + NT);
+    int* odd = reinterpret_cast<int*>(mean + NT);
+    for (int e = threadIdx.x; e < 2 * (kChunk + 1); e += blockDim.x) odd[e] = 0;
     __syncthreads();
 
-    auto yv = [&](int t, int n) -> double { return (double)ring[(t % L) * N + n] - mean[n]; };
+    // the tile: group (hemisphere with exc, else all nodes), row block, column
+    // block; only tiles with pairs j < i exist
+    const int M = a.exc ? a.N / 2 : a.N;
+    int tile = blockIdx.y, g0 = 0, bi = 0;
+    for (;; bi++) {
+        if (bi * TI >= M) {
+            g0 += M;
+            bi = 0;
+        }
+        const int imax = min((bi + 1) * TI, M) - 1, nb = imax < 1 ? 0 : (imax - 1) / TJ + 1;
+        if (tile < nb) break;
+        tile -= nb;
+    }
+    const int i0 = g0 + bi * TI, j0 = g0 + tile * TJ, gend = g0 + M;
+    const int N = a.N, L = a.win_len, T0 = a.corr_len, W = a.W, step = a.win_step, sim = blockIdx.x;
+    const TB* src = bold + ((size_t)sim * a.frames + a.n_vols_remove) * N;
+    const double invL = 1.0 / L, invT = 1.0 / T0;
+    const int chunks = (T0 + kChunk - 1) / kChunk;
+    int k = 0, lo = 0;  // current window and the first frame it covers
 
-    for (int t = 0; t < T0; t++) {
-        for (int n = threadIdx.x; n < N; n += blockDim.x) ring[(t % L) * N + n] = bold[base + (size_t)t * N + n];
-        __syncthreads();
-        const bool in_win = (k < a.W) && t >= lo;
-        for (int n = threadIdx.x; n < N; n += blockDim.x) {
-            const double y = yv(t, n);
-            fs[n] += y;
-            fss[n] += y * y;
-            if (in_win) {
-                ws[n] += y;
-                wss[n] += y * y;
-            }
-        }
+    if (threadIdx.x >= 256) {  // ---- one thread per node of the tile ----
+        const int n = threadIdx.x - 256;
+        const int node = n < TI ? i0 + n : j0 + n - TI;
+        const bool on = n < NT && node < gend;
+        const TB* x = src + (on ? node : i0);
+        double s = 0.0;
+        int t = 0;
+        for (; t + 8 <= T0; t += 8) {  // FP64 sum in frame order, eight loads in flight
+            TB v[8];
 #pragma unroll
-        for (int u = 0; u < PPT; u++) {
-            if (!pv[u]) continue;
-            const double yy = yv(t, pi[u]) * yv(t, pj[u]);
-            full[u] += yy;
-            if (in_win) win[u] += yy;
-        }
-        if (k < a.W && t == k * a.win_step + L - 1) {
-            __syncthreads();  // node window sums complete
-            const double invL = 1.0 / L;
+            for (int u = 0; u < 8; u++) v[u] = x[(size_t)(t + u) * N];
 #pragma unroll
-            for (int u = 0; u < PPT; u++) {
-                if (!pv[u]) continue;
-                const int i = pi[u], j = pj[u];
-                const double cov = win[u] - ws[i] * ws[j] * invL;
-                const double vi = wss[i] - ws[i] * ws[i] * invL;
-                const double vj = wss[j] - ws[j] * ws[j] * invL;
-                const double r = cov / sqrt(vi * vj);
-                const float rf = (float)r;
-                if (!(r == r) || isinf(r)) any_nan = true;
-                a.wfc[((size_t)sim * a.W + k) * a.P + p0 + u * blockDim.x + threadIdx.x] = rf;
-            }
-            __syncthreads();  // every pair has read this window's node sums
-            // slide to window k+1: drop the frames it no longer covers
-            const int nlo = (k + 1) * a.win_step;
-            if (nlo <= t) {
-                for (int tt = lo; tt < nlo; tt++) {
-                    for (int n = threadIdx.x; n < N; n += blockDim.x) {
-                        const double y = yv(tt, n);
-                        ws[n] -= y;
-                        wss[n] -= y * y;
+            for (int u = 0; u < 8; u++) s += (double)v[u];
+        }
+        for (; t < T0; t++) s += (double)x[(size_t)t * N];
+        const double mu = s / T0;
+        if (n < NT) mean[n] = mu;
+        double fs = 0.0, fss = 0.0, ws = 0.0, wss = 0.0;
+        TB v[kChunk];
+        auto fetch = [&](int c) {
+#pragma unroll
+            for (int f = 0; f < kChunk; f++) v[f] = x[(size_t)min(c * kChunk + f, T0 - 1) * N];
+        };
+        fetch(0);
+        int pos = 0;  // ring slot of frame t
+        for (int c = 0; c <= chunks; c++) {
+            if (c < chunks && n < NT) {
+                double y[kChunk];
+#pragma unroll
+                for (int f = 0; f < kChunk; f++) y[f] = (double)v[f] - mu;
+                if (c + 1 < chunks) fetch(c + 1);
+                int slot = 0;
+#pragma unroll
+                for (int f = 0; f < kChunk; f++) {
+                    const int t = c * kChunk + f;
+                    if (t >= T0) break;
+                    ring[pos * NT + n] = y[f];
+                    fs += y[f];
+                    fss = fma(y[f], y[f], fss);
+                    if (k < W && t >= lo) {
+                        ws += y[f];
+                        wss = fma(y[f], y[f], wss);
                     }
-#pragma unroll
-                    for (int u = 0; u < PPT; u++)
-                        if (pv[u]) win[u] -= yv(tt, pi[u]) * yv(tt, pj[u]);
+                    if (k < W && t == k * step + L - 1) {
+                        const double v = fma(-(ws * ws), invL, wss);
+                        stat[((c & 1) * kChunk + slot) * NT + n] = make_double2(ws, v);
+                        // a window's flag is never cleared: from then on its slot takes the plain path
+                        if (on && !var_ok(v)) odd[(c & 1) * kChunk + slot] = 1;
+                        slot++;
+                        // slide to window k + 1: drop the frames it no longer covers
+                        const int nlo = (k + 1) * step;
+                        if (nlo <= t) {
+                            for (int tt = lo; tt < nlo; tt++) {
+                                int q = pos - (t - tt);
+                                if (q < 0) q += rl;
+                                const double yl = kRing ? ring[q * NT + n] : (double)x[(size_t)tt * N] - mu;
+                                ws -= yl;
+                                wss = fma(-yl, yl, wss);
+                            }
+                        } else {
+                            ws = wss = 0.0;
+                        }
+                        lo = nlo;
+                        k++;
+                    }
+                    if (++pos == rl) pos = 0;
                 }
-            } else {
-                for (int n = threadIdx.x; n < N; n += blockDim.x) ws[n] = wss[n] = 0.0;
-#pragma unroll
-                for (int u = 0; u < PPT; u++) win[u] = 0.0;
+                if (c == chunks - 1) {
+                    const double v = fma(-(fs * fs), invT, fss);
+                    series[n] = make_double2(fs, v);
+                    if (on && !var_ok(v)) odd[2 * kChunk] = 1;
+                }
             }
-            lo = nlo;
-            k++;
+            __syncthreads();  // chunk c is ready, chunk c - 1 has been used
         }
-        __syncthreads();
+        return;
+    }
+
+    // ---- pairs ----
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    double full[RI][RJ], win[RI][RJ];
+    bool pv[RI][RJ];
+    int pidx[RI];  // pair index of (i, j) = pidx + j
+#pragma unroll
+    for (int u = 0; u < RI; u++) {
+        const int i = i0 + ty + 16 * u, r = i - g0;  // rows before i in its group hold r (r - 1) / 2 pairs
+        pidx[u] = (g0 ? M * (M - 1) / 2 : 0) + r * (r - 1) / 2 - g0;
+#pragma unroll
+        for (int w = 0; w < RJ; w++) {
+            pv[u][w] = i < gend && j0 + tx + 16 * w < i;
+            full[u][w] = win[u][w] = 0.0;
+        }
+    }
+    bool any_nan = false;
+    // correlations of the tile from co-moments m and node sums st, to `to`
+    auto emit = [&](const double (&m)[RI][RJ], const double2* st, double inv, bool plain, float* to) {
+        double2 si[RI], sj[RJ];
+#pragma unroll
+        for (int u = 0; u < RI; u++) si[u] = st[ty + 16 * u];
+#pragma unroll
+        for (int w = 0; w < RJ; w++) sj[w] = st[TI + tx + 16 * w];
+        unsigned again = 0;
+#pragma unroll
+        for (int u = 0; u < RI; u++)
+#pragma unroll
+            for (int w = 0; w < RJ; w++) {
+                bool redo;
+                const double cov = fma(-(si[u].x * sj[w].x), inv, m[u][w]);
+                const double r = corr_fast(cov, si[u].y, sj[w].y, redo);
+                if (pv[u][w]) to[pidx[u] + 16 * w] = (float)r;
+                again |= redo && pv[u][w] ? 1u << (u * RJ + w) : 0u;
+            }
+        if (!again && !plain) return;
+#pragma unroll
+        for (int u = 0; u < RI; u++)
+#pragma unroll
+            for (int w = 0; w < RJ; w++) {
+                if (!pv[u][w] || !(plain || (again >> (u * RJ + w) & 1))) continue;
+                const double cov = fma(-(si[u].x * sj[w].x), inv, m[u][w]);
+                const double r = corr_plain(cov, si[u].y, sj[w].y);
+                if (!(r == r) || isinf(r)) any_nan = true;
+                to[pidx[u] + 16 * w] = (float)r;
+            }
+    };
+    const double* yi = ring + ty;
+    const double* yj = ring + TI + tx;
+    float* out = a.wfc + (size_t)sim * W * a.P + j0 + tx;
+    __syncthreads();  // chunk 0
+    int pos = 0, lpos = 0;  // ring slots (as offsets) of frame t and of frame lo
+    const int rend = rl * NT;
+    int t_out = L - 1;  // last frame of window k
+    for (int c = 0; c < chunks; c++) {
+        int slot = (c & 1) * kChunk;
+        const int t1 = min(T0, (c + 1) * kChunk);
+        for (int t = c * kChunk; t < t1; t++) {
+            const bool in_win = k < W && t >= lo;
+            double ei[RI], ej[RJ];
+#pragma unroll
+            for (int u = 0; u < RI; u++) ei[u] = yi[pos + 16 * u];
+#pragma unroll
+            for (int w = 0; w < RJ; w++) ej[w] = yj[pos + 16 * w];
+#pragma unroll
+            for (int u = 0; u < RI; u++)
+#pragma unroll
+                for (int w = 0; w < RJ; w++) {
+                    full[u][w] = fma(ei[u], ej[w], full[u][w]);
+                    if (in_win) win[u][w] = fma(ei[u], ej[w], win[u][w]);
+                }
+            if (k < W && t == t_out) {
+                emit(win, stat + slot * NT, invL, odd[slot] != 0, out);
+                slot++;
+                out += a.P;
+                const int nlo = lo + step;
+                if (nlo <= t) {
+                    for (int tt = lo; tt < nlo; tt++) {
+                        double li[RI], lj[RJ];
+                        if (kRing) {
+#pragma unroll
+                            for (int u = 0; u < RI; u++) li[u] = yi[lpos + 16 * u];
+#pragma unroll
+                            for (int w = 0; w < RJ; w++) lj[w] = yj[lpos + 16 * w];
+                            lpos += NT;
+                            if (lpos == rend) lpos = 0;
+                        } else {
+                            const TB* x = src + (size_t)tt * N;
+#pragma unroll
+                            for (int u = 0; u < RI; u++)
+                                li[u] = (double)x[min(i0 + ty + 16 * u, gend - 1)] - mean[ty + 16 * u];
+#pragma unroll
+                            for (int w = 0; w < RJ; w++)
+                                lj[w] = (double)x[min(j0 + tx + 16 * w, gend - 1)] - mean[TI + tx + 16 * w];
+                        }
+#pragma unroll
+                        for (int u = 0; u < RI; u++)
+#pragma unroll
+                            for (int w = 0; w < RJ; w++) win[u][w] = fma(-li[u], lj[w], win[u][w]);
+                    }
+                } else {
+#pragma unroll
+                    for (int u = 0; u < RI; u++)
+#pragma unroll
+                        for (int w = 0; w < RJ; w++) win[u][w] = 0.0;
+                    if (kRing) lpos = nlo % rl * NT;
+                }
+                lo = nlo;
+                t_out += step;
+                k++;
+            }
+            pos += NT;
+            if (pos == rend) pos = 0;
+        }
+        __syncthreads();  // this chunk's ring slots and sums may be refilled
     }
     // static FC over all kept frames
-    const double invT = 1.0 / T0;
-#pragma unroll
-    for (int u = 0; u < PPT; u++) {
-        if (!pv[u]) continue;
-        const int i = pi[u], j = pj[u];
-        const double cov = full[u] - fs[i] * fs[j] * invT;
-        const double vi = fss[i] - fs[i] * fs[i] * invT;
-        const double vj = fss[j] - fs[j] * fs[j] * invT;
-        const double r = cov / sqrt(vi * vj);
-        if (!(r == r) || isinf(r)) any_nan = true;
-        a.fc[(size_t)sim * a.P + p0 + u * blockDim.x + threadIdx.x] = (float)r;
-    }
+    emit(full, series, invT, odd[2 * kChunk] != 0, a.fc + (size_t)sim * a.P + j0 + tx);
     if (any_nan) atomicOr(&a.nan_flag[sim], 1);
 }
 
@@ -346,29 +508,50 @@ __global__ void __launch_bounds__(1024) gof_kernel(GofArgs a) {
 
 using namespace bnm;
 
-template <typename TB, int PPT>
+template <typename TB, int RI, int RJ>
 static cudaError_t launch_fc_window_t(const FcArgs& a, const TB* bold, cudaStream_t st) {
-    constexpr int TPB = 256;
-    const int chunks = (a.P + TPB * PPT - 1) / (TPB * PPT);
-    const size_t smem = (size_t)a.N * 5 * sizeof(double) + (size_t)a.win_len * a.N * sizeof(TB);
-    if (smem > 227 * 1024) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(fc_window_kernel<TB, PPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr int TI = 16 * RI, TJ = 16 * RJ, NT = TI + TJ, threads = 256 + (RI + RJ + 1) / 2 * 32;
+    // window lengths are limited by what a ring of all nodes would take of one SM
+    if ((size_t)a.N * 5 * sizeof(double) + (size_t)a.win_len * a.N * sizeof(TB) > 227 * 1024) return cudaErrorInvalidValue;
+    const int M = a.exc ? a.N / 2 : a.N;
+    int tiles = 0;  // as the kernel counts them
+    for (int bi = 0; bi * TI < M; bi++) {
+        const int imax = std::min((bi + 1) * TI, M) - 1;
+        tiles += imax < 1 ? 0 : (imax - 1) / TJ + 1;
+    }
+    if (a.exc) tiles *= 2;
+    if (tiles < 1) return cudaErrorInvalidValue;
+    // the ring holds the window and two chunks where that leaves room for two
+    // CTAs an SM; else two chunks, and the frames that leave a window are read again
+    const size_t fixed = (size_t)2 * kChunk * NT * sizeof(double2) + NT * (sizeof(double2) + sizeof(double)) +
+                         2 * (kChunk + 1) * sizeof(int);
+    const int full = a.win_len + 2 * kChunk;
+    const bool ring = (size_t)full * NT * sizeof(double) + fixed <= 110 * 1024;
+    const int rl = ring ? full : 2 * kChunk;
+    const size_t smem = (size_t)rl * NT * sizeof(double) + fixed;
+    auto* fn = ring ? fc_window_kernel<TB, RI, RJ, true> : fc_window_kernel<TB, RI, RJ, false>;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    dim3 grid(a.n_sims, chunks);
-    fc_window_kernel<TB, PPT><<<grid, TPB, smem, st>>>(a, bold);
+    fn<<<dim3(a.n_sims, tiles), threads, smem, st>>>(a, bold, rl);
     return cudaGetLastError();
 }
 
-// The window tile: each CTA of 256 threads carries 256 ppt pairs through the
-// frames (ppt in {1, 2, 4, 8}); fewer pairs per CTA give more CTAs but repeat
-// the node means and the frame ring per CTA.  The plan's tuner picks ppt.
+// The window tile: each CTA of 256 pair threads carries 256 ppt pairs (nodes
+// 16 x 16, 16 x 32, 32 x 32 or 32 x 64) through the frames; fewer pairs per
+// CTA give more CTAs but repeat the nodes' series per CTA.  The plan's tuner
+// picks ppt; without one, the largest tile that still gives two CTAs an SM.
 template <typename TB>
 static cudaError_t launch_fc_window(const FcArgs& a, const TB* bold, cudaStream_t st) {
-    switch (a.ppt ? a.ppt : 4) {
-        case 1: return launch_fc_window_t<TB, 1>(a, bold, st);
-        case 2: return launch_fc_window_t<TB, 2>(a, bold, st);
-        case 4: return launch_fc_window_t<TB, 4>(a, bold, st);
-        case 8: return launch_fc_window_t<TB, 8>(a, bold, st);
+    int ppt = a.ppt;
+    if (!ppt) {
+        const long long ctas = (long long)a.P * a.n_sims / 256;  // of the smallest tile
+        ppt = ctas >= 8 * 300 ? 8 : ctas >= 4 * 300 ? 4 : ctas >= 2 * 300 ? 2 : 1;
+    }
+    switch (ppt) {
+        case 1: return launch_fc_window_t<TB, 1, 1>(a, bold, st);
+        case 2: return launch_fc_window_t<TB, 1, 2>(a, bold, st);
+        case 4: return launch_fc_window_t<TB, 2, 2>(a, bold, st);
+        case 8: return launch_fc_window_t<TB, 2, 4>(a, bold, st);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -142,7 +142,6 @@ struct bnm_plan {
     float* d_sc32 = nullptr;
     double *d_sc64 = nullptr, *d_sc_fic = nullptr;
     float* d_noise = nullptr;
-    int *d_pi = nullptr, *d_pj = nullptr;
     double *d_emp_fc = nullptr, *d_emp_sorted = nullptr;
     int* d_ks_lut = nullptr;
     unsigned char* d_valid = nullptr;
@@ -335,10 +334,6 @@ static int plan_create(const bnm_config* cfg, const double* sc, const double* em
             pi.push_back(i);
             pj.push_back(j);
         }
-    BNM_CUDA_TRY(dalloc(p, &p->d_pi, pi.size()));
-    BNM_CUDA_TRY(dalloc(p, &p->d_pj, pj.size()));
-    BNM_CUDA_TRY(cudaMemcpy(p->d_pi, pi.data(), pi.size() * 4, cudaMemcpyHostToDevice));
-    BNM_CUDA_TRY(cudaMemcpy(p->d_pj, pj.data(), pj.size() * 4, cudaMemcpyHostToDevice));
 
     // targets: empirical FC and its mean; empirical FCD sorted, with jump flags
     double mfc = 0;
@@ -633,8 +628,7 @@ static FcArgs fc_args(bnm_plan* p, int n) {
     fa.n_vols_remove = s.n_vols_remove;
     fa.corr_len = s.corr_len;
     fa.P = s.n_pairs;
-    fa.pair_i = p->d_pi;
-    fa.pair_j = p->d_pj;
+    fa.exc = c.exc_interhem;
     fa.W = c.no_fcd ? 0 : s.n_windows;
     fa.win_len = s.window_len;
     fa.win_step = c.window_step;

@@ -10,8 +10,7 @@ namespace bnm {
 struct FcArgs {
     int N, n_sims, frames, n_vols_remove, corr_len;
     int P;                    // pairs
-    const int* pair_i;        // [P]
-    const int* pair_j;        // [P]
+    int exc;                  // pairs within a hemisphere only
     int W, win_len, win_step; // windows: start k*step, length win_len (relative to first kept frame)
     const float* bold;        // [n][frames][N] (FP32 integrators)
     const double* bold_f64;   // [n][frames][N] (FP64 integrator); exactly one is set
@@ -19,7 +18,7 @@ struct FcArgs {
     float* wfc;               // [n][W][P] raw window FC
     double* wsum;             // [n][W][2] sum, sum of squares over pairs (written after the window FC)
     int* nan_flag;            // [n]
-    int ppt;                  // pairs per thread: a CTA of 256 threads covers 256 ppt pairs (0: 4)
+    int ppt;                  // pairs per thread: a CTA covers 256 ppt pairs (0: by the number of pairs)
 };
 
 struct FcdArgs {

@@ -57,31 +57,6 @@ int scratch_for(int device, unsigned char** out) {
     return BNM_OK;
 }
 
-// Lower-triangle pair table of run_CMAES.cpp:505-524 (i > j, i outer, j
-// inner; with exc_interhem the pairs that cross the N/2 split are skipped):
-// one thread per row i writes its pairs at the row's closed-form offset.
-__global__ void pair_table_kernel(int N, int exc, int* pi, int* pj) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const int h = N / 2;
-    long long start;
-    int j0;
-    if (!exc) {
-        start = (long long)i * (i - 1) / 2;
-        j0 = 0;
-    } else if (i < h) {
-        start = (long long)i * (i - 1) / 2;
-        j0 = 0;
-    } else {
-        start = (long long)h * (h - 1) / 2 + (long long)(i - h) * (i - h - 1) / 2;
-        j0 = h;
-    }
-    for (int j = j0; j < i; j++) {
-        pi[start + (j - j0)] = i;
-        pj[start + (j - j0)] = j;
-    }
-}
-
 // KS jump flags of the sorted empirical FCD: rank c (0..m) is a point where
 // F_emp jumps (c == 0, c == m, or e[c-1] < e[c]).
 __global__ void ks_valid_kernel(const double* e, int m, unsigned char* valid) {
@@ -127,7 +102,6 @@ extern "C" int bnm_gof_noalloc(const float* d_bold, int32_t n, int32_t frames, i
         off = align256(off + bytes);
         return at;
     };
-    const size_t o_pi = take((size_t)P * 4), o_pj = take((size_t)P * 4);
     const size_t o_efc = take((size_t)P * 8), o_es = take((size_t)m * 8), o_valid = take((size_t)m + 1);
     const size_t o_fc = take((size_t)n * P * 4), o_wfc = take((size_t)n * W * P * 4);
     const size_t o_wsum = take((size_t)n * W * 2 * 8), o_hist = take((size_t)n * (m + 1) * 4);
@@ -148,8 +122,6 @@ extern "C" int bnm_gof_noalloc(const float* d_bold, int32_t n, int32_t frames, i
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-    int* pi = reinterpret_cast<int*>(s + o_pi);
-    int* pj = reinterpret_cast<int*>(s + o_pj);
     double* efc = reinterpret_cast<double*>(s + o_efc);
     double* es = reinterpret_cast<double*>(s + o_es);
     unsigned char* valid = s + o_valid;
@@ -162,7 +134,6 @@ extern "C" int bnm_gof_noalloc(const float* d_bold, int32_t n, int32_t frames, i
     BNM_CUDA_TRY(cudaMemsetAsync(s + o_eq, 0, (size_t)n * (m + 1) * 4, st));
     BNM_CUDA_TRY(cudaMemsetAsync(s + o_nan, 0, (size_t)n * 4, st));
     BNM_CUDA_TRY(cudaMemsetAsync(s + o_zero, 0, 8 * (size_t)n + 8, st));
-    pair_table_kernel<<<(N + 127) / 128, 128, 0, st>>>(N, exc_interhem, pi, pj);
     ks_valid_kernel<<<(m + 256) / 256 < 1024 ? (m + 256) / 256 : 1024, 256, 0, st>>>(es, m, valid);
     BNM_CUDA_TRY(cudaGetLastError());
 
@@ -174,8 +145,7 @@ extern "C" int bnm_gof_noalloc(const float* d_bold, int32_t n, int32_t frames, i
     fa.n_vols_remove = n_vols_remove;
     fa.corr_len = corr_len;
     fa.P = P;
-    fa.pair_i = pi;
-    fa.pair_j = pj;
+    fa.exc = exc_interhem;
     fa.W = W;
     fa.win_len = L;
     fa.win_step = window_step;
