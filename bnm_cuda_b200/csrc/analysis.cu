@@ -22,11 +22,14 @@
 //     (64x64 output tiles, FP32), lower triangle only; its epilogue drops each
 //     FCD value into the KS histogram (upper_bound rank among the sorted
 //     empirical FCD), so FCD never has to be sorted.
-//   * gof_kernel: prefix-scan of that histogram gives the exact KS statistic;
+//   * gof_kernel: prefix-scan of that histogram (a cluster of CTAs per
+//     simulation) gives the exact KS statistic;
 //     FC correlation / mean difference in FP64; cost assembly.
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 #include <cuda_runtime.h>
+#include "cluster_util.cuh"
 #include "kernels.h"
 
 namespace bnm {
@@ -427,10 +430,80 @@ __device__ double block_max(double v, double* sh) {
     return s;
 }
 
+// One cluster of CTAs per simulation; every CTA takes a share of the KS bins
+// and every warp a contiguous piece of that, so the bins are read in whole
+// lines (one thread per contiguous piece of one CTA's bins read them 4 bytes
+// at a time at a stride of kilobytes: 0.90 ms for 4 simulations of 668,746
+// bins, 0.20 ms for 64 of 146,070; now 0.12 and 0.09 ms).  Rank 0 does the FC and the cost.
 __global__ void __launch_bounds__(1024) gof_kernel(GofArgs a) {
     __shared__ double sh[32];
-    __shared__ unsigned long long seg[1024];
-    const int sim = blockIdx.x;
+    __shared__ unsigned int wtot[32], total;  // FCD values counted in each warp's bins, in this CTA's
+    __shared__ double dks[8];                 // rank 0: every CTA's KS distance
+    const int rank = (int)cluster_rank(), ranks = (int)cluster_size();
+    const int sim = blockIdx.x / ranks, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (!a.no_fcd) {
+        // KS: D = max over jump points c of |c/m - F_sim| just before/at the point
+        const int nb = a.m + 1, nw = ranks * 32;
+        const unsigned int* h = a.hist + (size_t)sim * nb;
+        const unsigned int* q = a.eq + (size_t)sim * nb;
+        const int per = ((nb + nw - 1) / nw + 31) / 32 * 32;
+        const int c0 = min(nb, (rank * 32 + warp) * per), c1 = min(nb, c0 + per);
+        unsigned int loc = 0;
+#pragma unroll 4
+        for (int c = c0 + lane; c < c1; c += 32) loc += h[c];
+        loc = __reduce_add_sync(0xffffffffu, loc);
+        if (lane == 0) wtot[warp] = loc;
+        __syncthreads();
+        unsigned int H = __reduce_add_sync(0xffffffffu, lane < warp ? wtot[lane] : 0u);  // sims with rank < c0
+        if (threadIdx.x == 0) {
+            unsigned int t = 0;
+            for (int w = 0; w < 32; w++) t += wtot[w];
+            total = t;
+        }
+        cluster_sync();
+        for (int r = 0; r < rank; r++) H += ld_cluster_u32(map_rank(smem_u32(&total), (uint32_t)r));
+        const double invm = 1.0 / a.m, invn = 1.0 / a.n_fcd;
+        double dmax = 0.0;
+        constexpr int U = 4;  // lines of 32 bins in flight
+        for (int b = c0; b < c1; b += 32 * U) {
+            unsigned int hv[U], qv[U], inc[U];
+            bool ok[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int c = b + 32 * u + lane;
+                const bool in = c < c1;
+                hv[u] = in ? h[c] : 0u;
+                qv[u] = in ? q[c] : 0u;
+                ok[u] = in && a.valid[c];
+                inc[u] = hv[u];
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const unsigned int v = __shfl_up_sync(0xffffffffu, inc[u], o);
+                    if (lane >= o) inc[u] += v;
+                }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const unsigned int Hc = H + inc[u] - hv[u];  // sims with rank < c
+                const double Fe = (b + 32 * u + lane) * invm;
+                if (ok[u]) {
+                    dmax = fmax(dmax, fabs(Fe - (double)(Hc + qv[u]) * invn));
+                    dmax = fmax(dmax, fabs(Fe - (double)(Hc + hv[u]) * invn));
+                }
+                H += __shfl_sync(0xffffffffu, inc[u], 31);
+            }
+        }
+        const double D = block_max(dmax, sh);
+        if (threadIdx.x == 0) st_cluster_f64(map_rank(smem_u32(&dks[rank]), 0), D);
+    }
+    // also keeps every CTA's total in place until all have read it
+    cluster_sync();
+    if (rank != 0) return;
+    double D = 0.0;
+    if (!a.no_fcd)
+        for (int r = 0; r < ranks; r++) D = fmax(D, dks[r]);
     // FC: Pearson with the empirical FC, and mean difference (FP64, two passes)
     const float* fc = a.fc + (size_t)sim * a.P;
     double s = 0.0;
@@ -447,40 +520,6 @@ __global__ void __launch_bounds__(1024) gof_kernel(GofArgs a) {
     sxx = block_sum(sxx, sh);
     syy = block_sum(syy, sh);
     const double r = sxy / (sqrt(sxx) * sqrt(syy));
-    // KS: D = max over jump points c of |c/m - F_sim| just before/at the point
-    double D = 0.0;
-    if (!a.no_fcd) {
-        const int nb = a.m + 1;
-        const unsigned int* h = a.hist + (size_t)sim * nb;
-        const unsigned int* q = a.eq + (size_t)sim * nb;
-        const int per = (nb + blockDim.x - 1) / blockDim.x;
-        const int c0 = threadIdx.x * per, c1 = min(nb, c0 + per);
-        unsigned long long loc = 0;
-        for (int c = c0; c < c1; c++) loc += h[c];
-        seg[threadIdx.x] = loc;
-        __syncthreads();
-        if (threadIdx.x == 0) {  // exclusive scan of segment totals
-            unsigned long long run = 0;
-            for (int w = 0; w < (int)blockDim.x; w++) {
-                const unsigned long long v = seg[w];
-                seg[w] = run;
-                run += v;
-            }
-        }
-        __syncthreads();
-        unsigned long long H = seg[threadIdx.x];  // sims with rank < c0
-        const double invm = 1.0 / a.m, invn = 1.0 / a.n_fcd;
-        double dmax = 0.0;
-        for (int c = c0; c < c1; c++) {
-            const double Fe = c * invm;
-            if (a.valid[c]) {
-                dmax = fmax(dmax, fabs(Fe - (double)(H + q[c]) * invn));
-                dmax = fmax(dmax, fabs(Fe - (double)(H + h[c]) * invn));
-            }
-            H += h[c];
-        }
-        D = block_max(dmax, sh);
-    }
     double pen = 0.0;
     if (a.calc_fic_penalty) {
         double ps = 0.0;
@@ -611,6 +650,19 @@ cudaError_t bnm_launch_fcd(FcdArgs a, cudaStream_t st) {
 }
 
 cudaError_t bnm_launch_gof(const GofArgs& a, cudaStream_t st) {
-    gof_kernel<<<a.n_sims, 1024, 0, st>>>(a);
-    return cudaGetLastError();
+    // 8 CTAs a simulation where the bins are many; a small histogram (a warp
+    // then has fewer than four lines) is one CTA's
+    const int ranks = a.no_fcd || a.m < 4096 ? 1 : 8;
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof cfg);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ranks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(a.n_sims * ranks));
+    cfg.blockDim = dim3(1024);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.stream = st;
+    return cudaLaunchKernelEx(&cfg, gof_kernel, a);
 }
