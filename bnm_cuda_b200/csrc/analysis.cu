@@ -16,8 +16,8 @@
 //     pair keeps FP64 running co-moments, updated by one add and one subtract
 //     per frame as the window slides, so window FC costs O(P) per window
 //     instead of O(P*L).  Static FC comes from the same pass.  Window
-//     sums over pairs (for the FCD centring) follow in window_sums_kernel,
-//     FP64 in a fixed order, so the FCD does not depend on the window tile.
+//     sums over pairs (for the FCD centring) are formed from the finished rows
+//     in FP64 in a fixed order, so the FCD does not depend on the window tile.
 //   * fcd_gram_kernel: FCD = Z Z^T over the centred, unit-norm window-FC rows
 //     (64x64 output tiles, FP32), lower triangle only; its epilogue drops each
 //     FCD value into the KS histogram (upper_bound rank among the sorted
@@ -596,42 +596,22 @@ static cudaError_t launch_fc_window(const FcArgs& a, const TB* bold, cudaStream_
 }
 
 cudaError_t bnm_launch_fc_window(const FcArgs& a, cudaStream_t st) {
-    cudaError_t e = a.bold_f64 ? launch_fc_window<double>(a, a.bold_f64, st) : launch_fc_window<float>(a, a.bold, st);
-    if (e != cudaSuccess || a.W < 1) return e;
-    // The window rows' sums over all pairs, in a fixed order: the same BOLD
-    // gives the same FCD whatever the window tile and the launch order.
-    return bnm_launch_window_sums(a.wfc, a.n_sims, a.W, a.P, 0, a.P, a.wsum, st);
+    if (a.W >= 1 && a.P < 2) return cudaErrorInvalidValue;  // a window row of one value cannot be centred
+    return a.bold_f64 ? launch_fc_window<double>(a, a.bold_f64, st) : launch_fc_window<float>(a, a.bold, st);
 }
 
 // Window-FC sums over a pair range, one CTA per (window, simulation): the
-// centring of the hemisphere FCDs (window_fc_stats with save_hemis,
-// bnm.cu:436-496).
+// centring of fcd_gram_kernel's FCDs, over all pairs or (window_fc_stats with
+// save_hemis, bnm.cu:436-496) a hemisphere's.
 __global__ void __launch_bounds__(256) window_sums_kernel(const float* wfc, int W, int P, int p0, int p1,
                                                           double* out) {
     __shared__ double sh[16];
     const int w = blockIdx.x, sim = blockIdx.y;
-    const float* v = wfc + ((size_t)sim * W + w) * P;
-    double s = 0.0, ss = 0.0;
-    for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
-        const double x = v[p];
-        s += x;
-        ss += x * x;
-    }
-    s = warp_sum(s);
-    ss = warp_sum(ss);
-    if ((threadIdx.x & 31) == 0) {
-        sh[threadIdx.x >> 5] = s;
-        sh[8 + (threadIdx.x >> 5)] = ss;
-    }
-    __syncthreads();
+    double ws[2];
+    window_sums(wfc + ((size_t)sim * W + w) * P, p0, p1, sh, ws);
     if (threadIdx.x == 0) {
-        double a = 0.0, b = 0.0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) {
-            a += sh[k];
-            b += sh[8 + k];
-        }
-        out[((size_t)sim * W + w) * 2] = a;
-        out[((size_t)sim * W + w) * 2 + 1] = b;
+        out[((size_t)sim * W + w) * 2] = ws[0];
+        out[((size_t)sim * W + w) * 2 + 1] = ws[1];
     }
 }
 

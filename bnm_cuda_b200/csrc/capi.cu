@@ -636,7 +636,6 @@ static FcArgs fc_args(bnm_plan* p, int n) {
     fa.bold_f64 = p->d_bold64;
     fa.fc = p->d_fc;
     fa.wfc = p->d_wfc;
-    fa.wsum = p->d_wsum;
     fa.nan_flag = p->d_nan;
     return fa;
 }
@@ -681,8 +680,6 @@ static int tune_window(bnm_plan* p, int n) {
             else p->win_ppt = saved;
         }
     }
-    const size_t W = std::max(p->sz.n_windows, 1);
-    BNM_CUDA_TRY(cudaMemsetAsync(p->d_wsum, 0, (size_t)n * W * 2 * 8, p->st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_nan, 0, n * 4, p->st));
     p->win_tuned_n = n;
     return BNM_OK;
@@ -694,7 +691,7 @@ static int launch_analysis(bnm_plan* p, int n, int calc_fic_penalty, bool hemis)
     const int N = c.nodes;
     cudaStream_t st = p->st;
     p->n_gram = 0;
-    p->launches += c.no_fcd ? 2 : 3;  // window FC (+ window sums) and goodness of fit
+    p->launches += 2;  // window FC and goodness of fit
 
     BNM_CUDA_TRY(bnm_launch_fc_window(fc_args(p, n), st));
     const int split = c.gram == BNM_GRAM_BF16_SPLIT;
@@ -790,8 +787,9 @@ static int launch_analysis(bnm_plan* p, int n, int calc_fic_penalty, bool hemis)
         da.hist = p->d_hist;
         da.eq = p->d_eq;
         da.nan_flag = p->d_nan;
+        BNM_CUDA_TRY(bnm_launch_window_sums(p->d_wfc, n, s.n_windows, s.n_pairs, 0, s.n_pairs, p->d_wsum, st));
         BNM_CUDA_TRY(bnm_launch_fcd(da, st));
-        p->launches++;
+        p->launches += 2;
     }
     if (hemis) {
         // left / right hemisphere FCD over the first / last (N/2)(N/2-1)/2 pairs,
@@ -1140,7 +1138,6 @@ extern "C" int bnm_run(bnm_plan* p, int32_t n, const double* G, const double* w_
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_counter, 0, 16, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_status, 0, 16, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_nan, 0, n * 4, st));
-    BNM_CUDA_TRY(cudaMemsetAsync(p->d_wsum, 0, (size_t)n * std::max(s.n_windows, 1) * 2 * 8, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_hist, 0, (size_t)n * (p->m + 1) * 4, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_eq, 0, (size_t)n * (p->m + 1) * 4, st));
 
@@ -1203,7 +1200,6 @@ extern "C" int bnm_check_fit_bold(bnm_plan* p, int32_t n, const double* bold, bn
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_nan, 0, n * 4, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_failed, 0, n * 4, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_ext, 0, (size_t)n * 6 * N * 8, st));
-    BNM_CUDA_TRY(cudaMemsetAsync(p->d_wsum, 0, (size_t)n * std::max(s.n_windows, 1) * 2 * 8, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_hist, 0, (size_t)n * (p->m + 1) * 4, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_eq, 0, (size_t)n * (p->m + 1) * 4, st));
     for (int e = 0; e < 3; e++) BNM_CUDA_TRY(cudaEventRecord(p->ev[e], st));
@@ -1265,7 +1261,6 @@ static int enqueue_run(bnm_plan* p, int n) {
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_counter, 0, 16, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_status, 0, 16, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_nan, 0, n * 4, st));
-    BNM_CUDA_TRY(cudaMemsetAsync(p->d_wsum, 0, (size_t)n * std::max(s.n_windows, 1) * 2 * 8, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_hist, 0, (size_t)n * (p->m + 1) * 4, st));
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_eq, 0, (size_t)n * (p->m + 1) * 4, st));
     const SimArgs a = sim_args(p, n);

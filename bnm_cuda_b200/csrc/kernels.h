@@ -16,7 +16,6 @@ struct FcArgs {
     const double* bold_f64;   // [n][frames][N] (FP64 integrator); exactly one is set
     float* fc;                // [n][P]
     float* wfc;               // [n][W][P] raw window FC
-    double* wsum;             // [n][W][2] sum, sum of squares over pairs (written after the window FC)
     int* nan_flag;            // [n]
     int ppt;                  // pairs per thread: a CTA covers 256 ppt pairs (0: by the number of pairs)
 };
@@ -65,6 +64,47 @@ __device__ __forceinline__ void window_norm(const double* wsum, int P, double& m
     inv_ssd = 1.0 / sqrt(v);
 }
 
+// Sum and sum of squares of v[p0 .. p1) by a block of 256 threads, in a fixed
+// order: thread t adds v[p0 + t], v[p0 + t + 256], ...; then lanes by
+// butterfly, then warps.  Every thread gets both.  Sixteen loads are in flight
+// ahead of the additions.  sh: 16 doubles.
+__device__ __forceinline__ void window_sums(const float* v, int p0, int p1, double* sh, double (&out)[2]) {
+    constexpr int U = 16;
+    double s = 0.0, ss = 0.0;
+    int p = p0 + threadIdx.x;
+    for (; p + 256 * (U - 1) < p1; p += 256 * U) {
+        float x[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) x[u] = v[p + 256 * u];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const double d = x[u];
+            s += d;
+            ss = fma(d, d, ss);
+        }
+    }
+    for (; p < p1; p += 256) {
+        const double d = v[p];
+        s += d;
+        ss = fma(d, d, ss);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sh[threadIdx.x >> 5] = s;
+        sh[8 + (threadIdx.x >> 5)] = ss;
+    }
+    __syncthreads();
+    out[0] = out[1] = 0.0;
+    for (int k = 0; k < 8; k++) {
+        out[0] += sh[k];
+        out[1] += sh[8 + k];
+    }
+}
+
 // KS bucket of x: c = #emp <= x; also whether x equals emp[c-1].
 __device__ __forceinline__ void ks_bucket(const double* e, int m, double x, int& c, bool& equal) {
     int lo = 0, hi = m;  // upper_bound
@@ -108,7 +148,7 @@ constexpr int kGramTileRows = 128, kGramTileK = 64, kGramTileBytes = kGramTileRo
 struct OperandArgs {
     int n_sims, rows, K, row_blocks, kblocks;
     const float* wfc;         // FCD rows: [n][W][P] window FC ...
-    const double* wsum;       // ... and its [n][W][2] pair sums
+    double* wsum;             // ... and its [n][W][2] pair sums (written)
     const float* bold;        // FC rows: [n][frames][N] BOLD (FP32 integrators) ...
     const double* bold_f64;   // ... or FP64 (one of the two)
     int frames, n_vols_remove;
@@ -177,6 +217,7 @@ extern "C" int bnm_colsplit_shape(int N, int csize, int rpl, int k2, int krp, in
 extern "C" int bnm_colsplit_variants(int* out4, int max);
 extern "C" int bnm_cluster_shape(int N, int csize, int rpw, int kr, int* threads, int* rows, size_t* smem);
 cudaError_t bnm_launch_integrate_exact(const bnm::SimArgs& a, int fp64, int num_sms, cudaStream_t st);
+// Static and window FC.
 cudaError_t bnm_launch_fc_window(const bnm::FcArgs& a, cudaStream_t st);
 cudaError_t bnm_launch_fcd(bnm::FcdArgs a, cudaStream_t st);
 // Per-window sum and sum of squares of window FC over pairs [p0, p1) (FP64):

@@ -129,7 +129,6 @@ extern "C" int bnm_gof_noalloc(const float* d_bold, int32_t n, int32_t frames, i
     // previous call's contents)
     BNM_CUDA_TRY(cudaMemcpyAsync(efc, emp_fc, (size_t)P * 8, cudaMemcpyHostToDevice, st));
     BNM_CUDA_TRY(cudaMemcpyAsync(es, emp_fcd_sorted, (size_t)m * 8, cudaMemcpyHostToDevice, st));
-    BNM_CUDA_TRY(cudaMemsetAsync(s + o_wsum, 0, (size_t)n * W * 2 * 8, st));
     BNM_CUDA_TRY(cudaMemsetAsync(s + o_hist, 0, (size_t)n * (m + 1) * 4, st));
     BNM_CUDA_TRY(cudaMemsetAsync(s + o_eq, 0, (size_t)n * (m + 1) * 4, st));
     BNM_CUDA_TRY(cudaMemsetAsync(s + o_nan, 0, (size_t)n * 4, st));
@@ -153,9 +152,10 @@ extern "C" int bnm_gof_noalloc(const float* d_bold, int32_t n, int32_t frames, i
     fa.bold_f64 = nullptr;
     fa.fc = reinterpret_cast<float*>(s + o_fc);
     fa.wfc = reinterpret_cast<float*>(s + o_wfc);
-    fa.wsum = reinterpret_cast<double*>(s + o_wsum);
+    double* wsum = reinterpret_cast<double*>(s + o_wsum);
     fa.nan_flag = reinterpret_cast<int*>(s + o_nan);
     BNM_CUDA_TRY(bnm_launch_fc_window(fa, st));
+    BNM_CUDA_TRY(bnm_launch_window_sums(fa.wfc, n, W, P, 0, P, wsum, st));
 
     FcdArgs da;
     std::memset(&da, 0, sizeof da);  // no bucket table: plain rank search
@@ -163,7 +163,7 @@ extern "C" int bnm_gof_noalloc(const float* d_bold, int32_t n, int32_t frames, i
     da.W = W;
     da.P = P;
     da.wfc = fa.wfc;
-    da.wsum = fa.wsum;
+    da.wsum = wsum;
     da.fcd = nullptr;
     da.n_fcd = W * (W - 1) / 2;
     da.emp_sorted = es;
