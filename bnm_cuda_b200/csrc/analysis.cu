@@ -382,28 +382,22 @@ __global__ void __launch_bounds__(256) fcd_gram_kernel(FcdArgs a) {
     bool any_nan = false;
     unsigned int* hist = a.hist ? a.hist + (size_t)sim * (a.m + 1) : nullptr;
     unsigned int* eq = a.hist ? a.eq + (size_t)sim * (a.m + 1) : nullptr;
+    float x[16];
+    bool on[16];
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int wa = a0 + ty * 4 + i, wb = b0 + tx * 4 + j;
-            if (wa < a.W && wb < wa) {
-                const float v = acc[i][j];
-                if (!(v == v) || isinf(v)) { any_nan = true; continue; }
-                const size_t idx = (size_t)wa * (wa - 1) / 2 + wb;
-                if (a.fcd) a.fcd[(size_t)sim * a.n_fcd + idx] = v;
-                if (hist) {
-                    int c;
-                    bool equal;
-                    if (a.ks_lut)
-                        ks_bucket_lut(a.emp_sorted, a.ks_lut, a.m, (double)v, c, equal);
-                    else
-                        ks_bucket(a.emp_sorted, a.m, (double)v, c, equal);
-                    atomicAdd(&hist[c], 1u);
-                    if (equal) atomicAdd(&eq[c], 1u);
-                }
+            const int wa = a0 + ty * 4 + i, wb = b0 + tx * 4 + j, u = 4 * i + j;
+            x[u] = acc[i][j];
+            on[u] = wa < a.W && wb < wa;
+            if (on[u] && (!(x[u] == x[u]) || isinf(x[u]))) {
+                any_nan = true;
+                on[u] = false;
             }
+            if (on[u] && a.fcd) a.fcd[(size_t)sim * a.n_fcd + (size_t)wa * (wa - 1) / 2 + wb] = x[u];
         }
+    if (hist) ks_count<16>(a.emp_sorted, a.ks_lut, a.m, x, on, hist, eq);
     if (any_nan && a.nan_flag) atomicOr(&a.nan_flag[sim], 1);
 }
 

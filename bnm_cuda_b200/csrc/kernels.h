@@ -105,17 +105,6 @@ __device__ __forceinline__ void window_sums(const float* v, int p0, int p1, doub
     }
 }
 
-// KS bucket of x: c = #emp <= x; also whether x equals emp[c-1].
-__device__ __forceinline__ void ks_bucket(const double* e, int m, double x, int& c, bool& equal) {
-    int lo = 0, hi = m;  // upper_bound
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (e[mid] <= x) lo = mid + 1; else hi = mid;
-    }
-    c = lo;
-    equal = (c > 0) && (e[c - 1] == x);
-}
-
 // Bucket table over the sorted empirical FCD for the KS rank search: bucket b
 // covers [edge(b), edge(b+1)) with edge(b) = -1 + b 2^-15 (exact in double),
 // bucket 0 extends to -inf and the last to +inf; lut[b] = #emp < edge(b)
@@ -124,20 +113,57 @@ __device__ __forceinline__ void ks_bucket(const double* e, int m, double x, int&
 constexpr int kKsBuckets = 1 << 16;
 __host__ __device__ __forceinline__ double ks_edge(int b) { return -1.0 + b * (1.0 / 32768.0); }
 
-__device__ __forceinline__ void ks_bucket_lut(const double* e, const int* lut, int m, double x, int& c, bool& equal) {
+__device__ __forceinline__ int ks_bucket_of(double x) {
     const double t = (x + 1.0) * 32768.0;
     int b = t < 1.0 ? 0 : (t >= (double)(kKsBuckets - 1) ? kKsBuckets - 1 : (int)t);
     // x + 1 can round across an edge when |x| is tiny: settle b on the exact edges
     if (b > 0 && x < ks_edge(b)) b--;
     if (b < kKsBuckets - 1 && x >= ks_edge(b + 1)) b++;
-    int lo = lut[b], hi = lut[b + 1];
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (e[mid] <= x) lo = mid + 1; else hi = mid;
+    return b;
+}
+
+// Counts U values x (where on) into the KS histogram of the sorted empirical
+// FCD e[m]: rank c = #emp <= x in hist, and those that equal e[c-1] in eq.
+// lut: bucket table, or null for a plain search.  A rank is a chain of four or
+// five dependent loads, so the U searches go side by side.
+template <int U>
+__device__ __forceinline__ void ks_count(const double* e, const int* lut, int m, const float (&x)[U], const bool (&on)[U],
+                                         unsigned int* hist, unsigned int* eq) {
+    int lo[U], hi[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        lo[u] = hi[u] = 0;
+        if (!on[u]) continue;
+        const int b = ks_bucket_of((double)x[u]);
+        lo[u] = lut ? lut[b] : 0;
+        hi[u] = lut ? lut[b + 1] : m;
     }
-    c = lo;
-    equal = (c > 0) && (e[c - 1] == x);
-    (void)m;
+    for (bool more = true; more;) {  // upper_bound
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) v[u] = lo[u] < hi[u] ? e[(lo[u] + hi[u]) >> 1] : 0.0;
+        more = false;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int mid = (lo[u] + hi[u]) >> 1;
+            if (lo[u] < hi[u]) {
+                if (v[u] <= (double)x[u])
+                    lo[u] = mid + 1;
+                else
+                    hi[u] = mid;
+            }
+            more |= lo[u] < hi[u];
+        }
+    }
+    double last[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) last[u] = on[u] && lo[u] > 0 ? e[lo[u] - 1] : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        if (!on[u]) continue;
+        atomicAdd(&hist[lo[u]], 1u);
+        if (lo[u] > 0 && last[u] == (double)x[u]) atomicAdd(&eq[lo[u]], 1u);
+    }
 }
 
 // Tensor-core Gram operands: rows x K values as BF16 tiles of 128 rows x 64 K
