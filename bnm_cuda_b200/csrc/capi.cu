@@ -600,33 +600,36 @@ static int upload_params(bnm_plan* p, int n, const double* G, const double* w_ee
 // Autotuner of the FP32 integrator: times every candidate shape of
 // bnm_integrator_candidates on this batch size over 200 simulated
 // milliseconds without FIC (the per-millisecond cost does not depend on the
-// model time) and keeps the fastest.  With `share` (plans of a group, which
-// run side by side and split the SMs) the score is the time weighted by the
-// fraction of the GPU the launch fills (bnm_integrator_share): SM time, not
-// latency.  A plan keeps the shape of its first tuning for a batch size,
+// model time) and keeps the fastest.  For plans of a group, which run side by
+// side, `share` receives the shape with the least SM time instead: the time
+// weighted by the fraction of the GPU the launch fills (bnm_integrator_share);
+// group_shapes chooses.  A plan keeps the shape of its first tuning for a batch size,
 // whichever path ran it, so the same inputs give the same results through
 // bnm_run and through a group.  BNM_B200_SHAPE="kind,slots,csize,rpw,kr"
 // forces a shape; BNM_B200_SLOTS forces the register kernel's slots;
 // BNM_B200_TUNE=0 takes the first candidate untimed.
-static int tune_integrator(bnm_plan* p, const SimArgs& a, bool share = false) {
+static int tune_integrator(bnm_plan* p, const SimArgs& a, IntegratorShape* share = nullptr) {
     const int n = a.n_sims;
     if (p->tuned_n == n) return BNM_OK;
     IntegratorShape cand[128];
     const int nc = bnm_integrator_candidates(a.N, cand, 128);
     if (nc < 1) return fail(BNM_EINVAL, "no FP32 integrator for %d nodes", a.N);
     p->shape = cand[0];
+    if (share) *share = cand[0];
     p->n_tried = 0;
     if (const char* e = std::getenv("BNM_B200_SHAPE")) {
         IntegratorShape s{};
         if (std::sscanf(e, "%d,%d,%d,%d,%d", &s.kind, &s.slots, &s.csize, &s.rpw, &s.kr) != 5)
             return fail(BNM_EINVAL, "BNM_B200_SHAPE must be kind,slots,csize,rpw,kr");
         p->shape = s;
+        if (share) *share = s;
         p->tuned_n = n;
         return BNM_OK;
     }
     const char* slots = std::getenv("BNM_B200_SLOTS");
     if (slots && p->shape.kind == 0) {
         p->shape.slots = std::atoi(slots) == 2 ? 2 : 1;
+        if (share) *share = p->shape;
         p->tuned_n = n;
         return BNM_OK;
     }
@@ -640,7 +643,7 @@ static int tune_integrator(bnm_plan* p, const SimArgs& a, bool share = false) {
     t.adjust_fic = 0;
     t.order = nullptr;  // shapes are timed on claim order
     BNM_CUDA_TRY(cudaMemsetAsync(p->d_status, 0, 16, p->st));
-    double best = 1e300;
+    double best = 1e300, best_share = 1e300;
     for (int i = 0; i < nc; i++) {
         // shapes that integrate two particles together compute an idle one for a batch of one
         if (n < 2 && ((cand[i].kind == 0 && cand[i].slots == 2) || cand[i].kind == 4)) continue;
@@ -662,10 +665,14 @@ static int tune_integrator(bnm_plan* p, const SimArgs& a, bool share = false) {
         if (!ok) continue;
         BNM_CUDA_TRY(cudaEventElapsedTime(&ms, p->tev[0], p->tev[1]));
         p->n_tried++;
-        const double score = share ? ms * bnm_integrator_share(t, cand[i], p->num_sms) : ms;
-        if (score < best) {
-            best = score;
+        if (ms < best) {
+            best = ms;
             p->shape = cand[i];
+        }
+        const double sm = share ? ms * bnm_integrator_share(t, cand[i], p->num_sms) : 0.0;
+        if (share && sm < best_share) {
+            best_share = sm;
+            *share = cand[i];
         }
     }
     int status = 0;
@@ -1488,6 +1495,50 @@ static void set_order(bnm_group* g) {
     std::stable_sort(g->order.begin(), g->order.end(), [&](int a, int b) { return work[a] > work[b]; });
 }
 
+// CTAs of one integration.
+static int integrator_ctas(const IntegratorShape& s, int n, int num_sms) {
+    switch (s.kind) {
+        case 0: return (n + s.slots - 1) / s.slots;
+        case 1:
+        case 3: return n * s.csize;
+        case 4: return (n + 1) / 2 * s.csize;
+        default: return std::min(n, 2 * num_sms);
+    }
+}
+
+// Tunes the plans of a group that have no shape for their batch sizes yet.
+// While the fastest shapes of all plans leave every CTA an SM of its own, the
+// plans do not take SMs from one another and the fastest shapes are kept;
+// otherwise each plan gets the shape with the least SM time.  (Two subjects
+// of 68 and 84 nodes, 32 particles each: by SM time the second ran two
+// particles per CTA on a GPU with 84 idle SMs, 543 ms a generation; 286 ms by
+// time.)
+static int group_shapes(bnm_group* g) {
+    const size_t np = g->plans.size();
+    std::vector<IntegratorShape> share(np);
+    std::vector<char> fresh(np, 0);
+    long long ctas = 0;
+    int rc;
+    for (size_t i = 0; i < np; i++) {
+        bnm_plan* p = g->plans[i];
+        if (p->cfg.precision != BNM_PREC_F32) {
+            ctas += std::min(g->n[i], 2 * p->num_sms);
+            continue;
+        }
+        BNM_CUDA_TRY(cudaMemcpy(p->d_G, p->io_G, g->n[i] * 8, cudaMemcpyHostToDevice));
+        BNM_CUDA_TRY(cudaMemcpy(p->d_wEE, p->io_wEE, (size_t)g->n[i] * p->cfg.nodes * 8, cudaMemcpyHostToDevice));
+        BNM_CUDA_TRY(cudaMemcpy(p->d_wEI, p->io_wEI, (size_t)g->n[i] * p->cfg.nodes * 8, cudaMemcpyHostToDevice));
+        if ((rc = launch_fic(p, g->n[i]))) return rc;
+        fresh[i] = p->tuned_n != g->n[i];
+        if ((rc = tune_integrator(p, sim_args(p, g->n[i]), np > 1 ? &share[i] : nullptr))) return rc;
+        ctas += integrator_ctas(p->shape, g->n[i], p->num_sms);
+    }
+    if (np > 1 && ctas > g->plans[0]->num_sms)
+        for (size_t i = 0; i < np; i++)
+            if (fresh[i]) g->plans[i]->shape = share[i];
+    return BNM_OK;
+}
+
 static int capture(bnm_group* g) {
     if (g->exec) cudaGraphExecDestroy(g->exec);
     if (g->graph) cudaGraphDestroy(g->graph);
@@ -1552,17 +1603,9 @@ extern "C" int bnm_group_run(bnm_group* g, const int32_t* n, const double* const
         // plan's integrator, which a capture cannot do), then capture the graph
         g->n = sizes;
         set_order(g);
-        for (size_t i = 0; i < np; i++) {
-            bnm_plan* p = g->plans[i];
-            if (p->cfg.precision == BNM_PREC_F32) {
-                BNM_CUDA_TRY(cudaMemcpy(p->d_G, p->io_G, sizes[i] * 8, cudaMemcpyHostToDevice));
-                BNM_CUDA_TRY(cudaMemcpy(p->d_wEE, p->io_wEE, (size_t)sizes[i] * p->cfg.nodes * 8, cudaMemcpyHostToDevice));
-                BNM_CUDA_TRY(cudaMemcpy(p->d_wEI, p->io_wEI, (size_t)sizes[i] * p->cfg.nodes * 8, cudaMemcpyHostToDevice));
-                if ((rc = launch_fic(p, sizes[i]))) return rc;
-                if ((rc = tune_integrator(p, sim_args(p, sizes[i]), np > 1))) return rc;
-            }
-            if ((rc = tune_window(p, sizes[i]))) return rc;
-        }
+        if ((rc = group_shapes(g))) return rc;
+        for (size_t i = 0; i < np; i++)
+            if ((rc = tune_window(g->plans[i], sizes[i]))) return rc;
         BNM_CUDA_TRY(cudaEventRecord(g->t0, g->origin));
         BNM_CUDA_TRY(cudaEventRecord(g->fork, g->origin));
         for (size_t k = 0; k < np; k++) {

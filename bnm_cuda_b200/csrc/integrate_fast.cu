@@ -503,54 +503,52 @@ static size_t fast_smem(int N, int threads) {
            (1 + P * kStages) * sizeof(uint64_t);
 }
 
-template <int K, int KC, int P>
-static cudaError_t launch_fast(const SimArgs& a, int grid, cudaStream_t st) {
-    const int threads = ((a.N + 31) / 32) * 32;
-    if (!a.noise) {  // noise drawn in the kernel
-        const size_t smem = fast_smem<K, KC, P, true>(a.N, threads);
-        cudaError_t e = cudaFuncSetAttribute(integrate_fast_kernel<K, KC, P, true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        integrate_fast_kernel<K, KC, P, true><<<grid, threads, smem, st>>>(a);
-        return cudaGetLastError();
+// CTAs of one variant that an SM holds at once (0 on error).
+template <typename F>
+static int fast_resident(F* fn, int threads, size_t smem) {
+    int per_sm = 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
     }
-    const size_t smem = fast_smem<K, KC, P, false>(a.N, threads);
-    if constexpr (P == 1) {
-        if (a.order) {  // placement
-            cudaError_t e = cudaFuncSetAttribute(integrate_fast_kernel<K, KC, 1, false, true>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-            integrate_fast_kernel<K, KC, 1, false, true><<<grid, threads, smem, st>>>(a);
-            return cudaGetLastError();
-        }
-    }
-    cudaError_t e = cudaFuncSetAttribute(integrate_fast_kernel<K, KC, P, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    integrate_fast_kernel<K, KC, P, false><<<grid, threads, smem, st>>>(a);
+    return per_sm;
+}
+
+// CTAs are persistent over the batch, as many as the GPU holds at once.  (For
+// 300 particles at N = 83, three CTAs an SM give 64 ms, as two at most did with
+// 4 particles in a second round: two CTAs fill an SM's issue slots.)
+template <int K, int KC, int P, bool NZI, bool PL = false>
+static cudaError_t launch_fast_t(const SimArgs& a, int num_sms, cudaStream_t st) {
+    const int threads = ((a.N + 31) / 32) * 32, need = (a.n_sims + P - 1) / P;
+    const size_t smem = fast_smem<K, KC, P, NZI>(a.N, threads);
+    auto* fn = integrate_fast_kernel<K, KC, P, NZI, PL>;
+    const int per_sm = fast_resident(fn, threads, smem);
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    const int grid = need < per_sm * num_sms ? need : per_sm * num_sms;
+    fn<<<grid, threads, smem, st>>>(a);
     return cudaGetLastError();
 }
 
+template <int K, int KC, int P>
+static cudaError_t launch_fast(const SimArgs& a, int num_sms, cudaStream_t st) {
+    if (!a.noise) return launch_fast_t<K, KC, P, true>(a, num_sms, st);  // noise drawn in the kernel
+    if constexpr (P == 1)
+        if (a.order) return launch_fast_t<K, KC, 1, false, true>(a, num_sms, st);  // placement
+    return launch_fast_t<K, KC, P, false>(a, num_sms, st);
+}
+
 template <int K, int KC, int P, bool NZI>
-static double share_fast_t(const SimArgs& a, int grid, int num_sms) {
-    const int threads = ((a.N + 31) / 32) * 32;
-    const size_t smem = fast_smem<K, KC, P, NZI>(a.N, threads);
-    int per_sm = 0;
-    if (cudaFuncSetAttribute(integrate_fast_kernel<K, KC, P, NZI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, integrate_fast_kernel<K, KC, P, NZI>, threads, smem) !=
-            cudaSuccess ||
-        per_sm < 1) {
-        cudaGetLastError();
-        return 1.0;
-    }
-    const double cap = (double)per_sm * num_sms;
-    return grid >= cap ? 1.0 : grid / cap;
+static double share_fast_t(const SimArgs& a, int num_sms) {
+    const int threads = ((a.N + 31) / 32) * 32, need = (a.n_sims + P - 1) / P;
+    const int cap = fast_resident(integrate_fast_kernel<K, KC, P, NZI>, threads, fast_smem<K, KC, P, NZI>(a.N, threads)) *
+                    num_sms;
+    return cap < 1 || need >= cap ? 1.0 : (double)need / cap;
 }
 
 template <int K, int KC, int P>
-static double share_fast(const SimArgs& a, int grid, int num_sms) {
-    return a.noise ? share_fast_t<K, KC, P, false>(a, grid, num_sms) : share_fast_t<K, KC, P, true>(a, grid, num_sms);
+static double share_fast(const SimArgs& a, int num_sms) {
+    return a.noise ? share_fast_t<K, KC, P, false>(a, num_sms) : share_fast_t<K, KC, P, true>(a, num_sms);
 }
 
 }  // namespace bnm
@@ -574,18 +572,14 @@ cudaError_t bnm_launch_integrate_shape(const bnm::SimArgs& a, const bnm::Integra
         const int ld = bnm_fast_kmax(a.N);
         if (!ld || a.sc_ld != ld || (sh.slots != 1 && sh.slots != 2)) return cudaErrorInvalidValue;
         if (a.noise && a.noise_ld != a.N) return cudaErrorInvalidValue;
-        // CTAs are persistent over the batch: two per SM with one slot, one with two
         const int P = sh.slots;
-        int grid = (a.n_sims + P - 1) / P;
-        const int max_grid = P == 1 ? 2 * num_sms : num_sms;
-        if (grid > max_grid) grid = max_grid;
         const int kc = fast_kc(a.N);
         switch ((ld / 4) * 8 + (ld / 4 - kc) * 2 + P) {
 #define BNM_K(K)                                                            \
-    case K * 8 + 1: return launch_fast<K, K, 1>(a, grid, st);            \
-    case K * 8 + 2: return launch_fast<K, K, 2>(a, grid, st);            \
-    case K * 8 + 4 + 1: return launch_fast<K, K - 2, 1>(a, grid, st); \
-    case K * 8 + 4 + 2: return launch_fast<K, K - 2, 2>(a, grid, st);
+    case K * 8 + 1: return launch_fast<K, K, 1>(a, num_sms, st);            \
+    case K * 8 + 2: return launch_fast<K, K, 2>(a, num_sms, st);            \
+    case K * 8 + 4 + 1: return launch_fast<K, K - 2, 1>(a, num_sms, st); \
+    case K * 8 + 4 + 2: return launch_fast<K, K - 2, 2>(a, num_sms, st);
             BNM_K(4) BNM_K(8) BNM_K(12) BNM_K(16) BNM_K(20) BNM_K(24) BNM_K(28) BNM_K(32)
 #undef BNM_K
             default: return cudaErrorInvalidValue;
@@ -613,16 +607,13 @@ double bnm_integrator_share(const bnm::SimArgs& a, const bnm::IntegratorShape& s
         const int ld = bnm_fast_kmax(a.N);
         if (!ld || (sh.slots != 1 && sh.slots != 2)) return 1.0;
         const int P = sh.slots;
-        int grid = (a.n_sims + P - 1) / P;
-        const int max_grid = P == 1 ? 2 * num_sms : num_sms;
-        if (grid > max_grid) grid = max_grid;
         const int kc = fast_kc(a.N);
         switch ((ld / 4) * 8 + (ld / 4 - kc) * 2 + P) {
 #define BNM_K(K)                                                                  \
-    case K * 8 + 1: return share_fast<K, K, 1>(a, grid, num_sms);              \
-    case K * 8 + 2: return share_fast<K, K, 2>(a, grid, num_sms);              \
-    case K * 8 + 4 + 1: return share_fast<K, K - 2, 1>(a, grid, num_sms); \
-    case K * 8 + 4 + 2: return share_fast<K, K - 2, 2>(a, grid, num_sms);
+    case K * 8 + 1: return share_fast<K, K, 1>(a, num_sms);              \
+    case K * 8 + 2: return share_fast<K, K, 2>(a, num_sms);              \
+    case K * 8 + 4 + 1: return share_fast<K, K - 2, 1>(a, num_sms); \
+    case K * 8 + 4 + 2: return share_fast<K, K - 2, 2>(a, num_sms);
             BNM_K(4) BNM_K(8) BNM_K(12) BNM_K(16) BNM_K(20) BNM_K(24) BNM_K(28) BNM_K(32)
 #undef BNM_K
             default: return 1.0;
