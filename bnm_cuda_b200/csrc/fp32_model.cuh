@@ -114,32 +114,54 @@ __device__ __forceinline__ float log1p_bw(float x) {
 // (log1p / expm1 through log1p_bw / expm1_bw).
 struct BW {
     float x = 0.f, ft = 0.f, nt = 0.f, qt = 0.f, lnu = 0.f;  // lnu = log(nu) = log1p(nt)
-    __device__ __forceinline__ void step(float S_E) {
-        typedef Model<float> C;
-        const float L1mr = -0.41551544396166582f;  // ln(1 - rho)
-        const float a1 = C::ialpha - 1.0f;         // exponent of nu in nu^(1/alpha) q / nu
-        x = x + C::model_dt * (S_E - C::kappa * x - C::y * ft);
-        const float ft_new = ft + C::model_dt * x;
-        const float pw = expm1_bw(C::ialpha * lnu);  // nu^(1/alpha) - 1, old nu
-        const float nt_new = nt + C::model_dt * C::itau * (ft - pw);
-        // f (1 - (1-rho)^(1/f)) / rho - 1, without cancellation:
-        // 1 - (1-rho)^(1/f) - rho = -(1-rho) expm1(ln(1-rho) (1/f - 1))
-        const float h = -(1.0f - C::rho) * expm1_bw(-L1mr * __fdividef(ft, 1.0f + ft));
-        const float inflow = (h + ft * (C::rho + h)) * (1.0f / C::rho);
-        // nu^(1/alpha - 1) q - 1 with the updated nu
-        const float lnu_new = log1p_bw(nt_new);
-        const float e = expm1_bw(a1 * lnu_new);
-        const float outflow = e + qt * (1.0f + e);
-        qt = qt + C::model_dt * C::itau * (inflow - outflow);
-        nt = nt_new;
-        lnu = lnu_new;
-        ft = ft_new;
-    }
+    __device__ __forceinline__ void step(float S_E);
     __device__ __forceinline__ float bold() const {
         typedef Model<float> C;
         // V0 (k1 (1-q) + k2 (1 - q/nu) + k3 (1-nu))
         return C::V_0 * (-C::k1 * qt + C::k2 * (nt - qt) / (1.0f + nt) - C::k3 * nt);
     }
 };
+
+// One step of BW in four pieces, for kernels that do it between other work;
+// BW::step is all of them.
+struct BWStep {
+    float x_new, ft_new, nt_new, in, lnu_new;
+    __device__ __forceinline__ void begin(const BW& b, float S_E) {
+        typedef Model<float> C;
+        x_new = b.x + C::model_dt * (S_E - C::kappa * b.x - C::y * b.ft);
+        ft_new = b.ft + C::model_dt * x_new;
+        const float pw = expm1_bw(C::ialpha * b.lnu);  // nu^(1/alpha) - 1, old nu
+        nt_new = b.nt + C::model_dt * C::itau * (b.ft - pw);
+    }
+    __device__ __forceinline__ void inflow(const BW& b) {
+        typedef Model<float> C;
+        const float L1mr = -0.41551544396166582f;  // ln(1 - rho)
+        // f (1 - (1-rho)^(1/f)) / rho - 1, without cancellation:
+        // 1 - (1-rho)^(1/f) - rho = -(1-rho) expm1(ln(1-rho) (1/f - 1))
+        const float h = -(1.0f - C::rho) * expm1_bw(-L1mr * __fdividef(b.ft, 1.0f + b.ft));
+        in = (h + b.ft * (C::rho + h)) * (1.0f / C::rho);
+    }
+    __device__ __forceinline__ void volume(const BW&) { lnu_new = log1p_bw(nt_new); }
+    __device__ __forceinline__ void end(BW& b, bool take = true) {  // take: else the step is dropped
+        typedef Model<float> C;
+        const float a1 = C::ialpha - 1.0f;  // exponent of nu in nu^(1/alpha) q / nu
+        // nu^(1/alpha - 1) q - 1 with the updated nu
+        const float e = expm1_bw(a1 * lnu_new);
+        const float outflow = e + b.qt * (1.0f + e);
+        const float qt_new = b.qt + C::model_dt * C::itau * (in - outflow);
+        b.x = take ? x_new : b.x;
+        b.qt = take ? qt_new : b.qt;
+        b.nt = take ? nt_new : b.nt;
+        b.lnu = take ? lnu_new : b.lnu;
+        b.ft = take ? ft_new : b.ft;
+    }
+};
+__device__ __forceinline__ void BW::step(float S_E) {
+    BWStep s;
+    s.begin(*this, S_E);
+    s.inflow(*this);
+    s.volume(*this);
+    s.end(*this);
+}
 
 }  // namespace bnm
