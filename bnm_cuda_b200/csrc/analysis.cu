@@ -19,7 +19,7 @@
 //     sums over pairs (for the FCD centring) are formed from the finished rows
 //     in FP64 in a fixed order, so the FCD does not depend on the window tile.
 //   * fcd_gram_kernel: FCD = Z Z^T over the centred, unit-norm window-FC rows
-//     (64x64 output tiles, FP32), lower triangle only; its epilogue drops each
+//     (FP32), lower triangle only; its epilogue drops each
 //     FCD value into the KS histogram (upper_bound rank among the sorted
 //     empirical FCD), so FCD never has to be sorted.
 //   * gof_kernel: prefix-scan of that histogram (a cluster of CTAs per
@@ -319,16 +319,25 @@ __global__ void __launch_bounds__(256 + (RI + RJ + 1) / 2 * 32) fc_window_kernel
 
 // ---------------------------------------------------------------- FCD Gram
 
-constexpr int kTile = 64, kTk = 16;
+// kTile x kTile outputs per CTA, RT x RT per thread (16 x 16 threads).  K
+// chunks are normalised (FP64) into one of two shared buffers while the other
+// is used, their loads in flight a chunk ahead.  Every output's sum runs over
+// K in order.  Few simulations with few windows leave most SMs without a
+// 64 x 64 tile (4 x 121 windows of 1122 pairs: 12 CTAs, 230 us with one buffer
+// and no load ahead), so those take 32 x 32 (40 CTAs, 54 us); many take the
+// larger tile, which reads each row half as often.
+constexpr int kTk = 32;
 
+template <int kTile>
 __global__ void __launch_bounds__(256) fcd_gram_kernel(FcdArgs a) {
+    constexpr int RT = kTile / 16, kLoads = kTile * kTk / 256;
     // blockIdx.x: lower-triangular tile index, blockIdx.y: simulation
     int t = blockIdx.x, ta = 0;
     while (t >= ta + 1) { t -= ta + 1; ta++; }
     const int tb = t;  // ta >= tb
     const int sim = blockIdx.y;
-    __shared__ float As[kTk][kTile + 4];
-    __shared__ float Bs[kTk][kTile + 4];
+    __shared__ float As[2][kTk][kTile + 1];
+    __shared__ float Bs[2][kTk][kTile + 1];
     __shared__ double mA[kTile], sA[kTile], mB[kTile], sB[kTile];
     const int a0 = ta * kTile, b0 = tb * kTile;
     const float* V = a.wfc + (size_t)sim * a.W * a.P;
@@ -347,48 +356,65 @@ __global__ void __launch_bounds__(256) fcd_gram_kernel(FcdArgs a) {
         sB[threadIdx.x - kTile] = s;
     }
     __syncthreads();
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16x16 threads, 4x4 outputs each
-    float acc[4][4];
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    const int lc = threadIdx.x % kTk, lr = threadIdx.x / kTk;  // column of this thread's loads, first row
+    constexpr int kStep = 256 / kTk;
+    float va[kLoads], vb[kLoads];
+    auto fetch = [&](int k0) {
+        const int col = k0 + lc;
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-    for (int k0 = a.p0; k0 < a.p1; k0 += kTk) {
-        // load 64 rows x 16 columns of A and B, normalised on the fly
-        for (int e = threadIdx.x; e < kTile * kTk; e += blockDim.x) {
-            const int r = e / kTk, c = e % kTk;
-            const int ra = a0 + r, rb = b0 + r, col = k0 + c;
-            float va = 0.f, vb = 0.f;
-            if (ra < a.W && col < a.p1) va = (float)(((double)V[(size_t)ra * a.P + col] - mA[r]) * sA[r]);
-            if (rb < a.W && col < a.p1) vb = (float)(((double)V[(size_t)rb * a.P + col] - mB[r]) * sB[r]);
-            As[c][r] = va;
-            Bs[c][r] = vb;
+        for (int e = 0; e < kLoads; e++) {
+            const int ra = a0 + lr + e * kStep, rb = b0 + lr + e * kStep;
+            va[e] = ra < a.W && col < a.p1 ? V[(size_t)ra * a.P + col] : 0.f;
+            vb[e] = rb < a.W && col < a.p1 ? V[(size_t)rb * a.P + col] : 0.f;
         }
-        __syncthreads();
+    };
+    auto store = [&](int buf, int k0) {  // centred and scaled; zero outside the rows and the pair range
+        const int col = k0 + lc;
 #pragma unroll
+        for (int e = 0; e < kLoads; e++) {
+            const int r = lr + e * kStep;
+            As[buf][lc][r] = a0 + r < a.W && col < a.p1 ? (float)(((double)va[e] - mA[r]) * sA[r]) : 0.f;
+            Bs[buf][lc][r] = b0 + r < a.W && col < a.p1 ? (float)(((double)vb[e] - mB[r]) * sB[r]) : 0.f;
+        }
+    };
+    float acc[RT][RT];
+#pragma unroll
+    for (int i = 0; i < RT; i++)
+#pragma unroll
+        for (int j = 0; j < RT; j++) acc[i][j] = 0.f;
+    fetch(a.p0);
+    store(0, a.p0);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = a.p0; k0 < a.p1; k0 += kTk, buf ^= 1) {
+        const bool more = k0 + kTk < a.p1;
+        if (more) fetch(k0 + kTk);
+#pragma unroll 8
         for (int c = 0; c < kTk; c++) {
-            float av[4], bv[4];
+            float av[RT], bv[RT];
 #pragma unroll
-            for (int i = 0; i < 4; i++) av[i] = As[c][ty * 4 + i];
+            for (int i = 0; i < RT; i++) av[i] = As[buf][c][ty * RT + i];
 #pragma unroll
-            for (int j = 0; j < 4; j++) bv[j] = Bs[c][tx * 4 + j];
+            for (int j = 0; j < RT; j++) bv[j] = Bs[buf][c][tx + 16 * j];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < RT; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+                for (int j = 0; j < RT; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
         }
+        if (more) store(buf ^ 1, k0 + kTk);
         __syncthreads();
     }
     bool any_nan = false;
     unsigned int* hist = a.hist ? a.hist + (size_t)sim * (a.m + 1) : nullptr;
     unsigned int* eq = a.hist ? a.eq + (size_t)sim * (a.m + 1) : nullptr;
-    float x[16];
-    bool on[16];
+    float x[RT * RT];
+    bool on[RT * RT];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < RT; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int wa = a0 + ty * 4 + i, wb = b0 + tx * 4 + j, u = 4 * i + j;
+        for (int j = 0; j < RT; j++) {
+            const int wa = a0 + ty * RT + i, wb = b0 + tx + 16 * j, u = RT * i + j;
             x[u] = acc[i][j];
             on[u] = wa < a.W && wb < wa;
             if (on[u] && (!(x[u] == x[u]) || isinf(x[u]))) {
@@ -397,7 +423,7 @@ __global__ void __launch_bounds__(256) fcd_gram_kernel(FcdArgs a) {
             }
             if (on[u] && a.fcd) a.fcd[(size_t)sim * a.n_fcd + (size_t)wa * (wa - 1) / 2 + wb] = x[u];
         }
-    if (hist) ks_count<16>(a.emp_sorted, a.ks_lut, a.m, x, on, hist, eq);
+    if (hist) ks_count<RT * RT>(a.emp_sorted, a.ks_lut, a.m, x, on, hist, eq);
     if (any_nan && a.nan_flag) atomicOr(&a.nan_flag[sim], 1);
 }
 
@@ -616,10 +642,16 @@ cudaError_t bnm_launch_window_sums(const float* wfc, int n_sims, int W, int P, i
     return cudaGetLastError();
 }
 
-cudaError_t bnm_launch_fcd(FcdArgs a, cudaStream_t st) {
-    a.tiles = (a.W + kTile - 1) / kTile;
-    dim3 grid(a.tiles * (a.tiles + 1) / 2, a.n_sims);
-    fcd_gram_kernel<<<grid, 256, 0, st>>>(a);
+cudaError_t bnm_launch_fcd(const FcdArgs& a, cudaStream_t st) {
+    auto tiles = [&](int tile) {
+        const int side = (a.W + tile - 1) / tile;
+        return side * (side + 1) / 2;
+    };
+    // the larger tile from two CTAs an SM on
+    if ((long long)tiles(64) * a.n_sims >= 296)
+        fcd_gram_kernel<64><<<dim3(tiles(64), a.n_sims), 256, 0, st>>>(a);
+    else
+        fcd_gram_kernel<32><<<dim3(tiles(32), a.n_sims), 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 
