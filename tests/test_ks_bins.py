@@ -29,3 +29,20 @@ def test_ks_matches_oracle(port, m):
     for i in range(n):
         # of the device's own FCD: counts over lengths, exact up to the last ulp
         assert r["fcd_ks"][i] == pytest.approx(port.port_ks(np.sort(emp), r["fcd"][i]), abs=1e-12)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [600, 70000])
+def test_graph_launch_counts_the_same(m):
+    rng = np.random.default_rng(m)
+    N, n = 12, 4
+    cfg = B.Config(nodes=N, max_sims=n, time_steps=4000, bold_tr=100, bold_remove_s=1, window_size=8, window_step=1,
+                   exc_interhem=False, i_sampling_start=100, i_sampling_end=600)
+    G, w = rng.uniform(0.5, 3, n), rng.uniform(0.1, 0.7, (n, N))
+    with B.Plan(cfg, rng.random((N, N)) * 0.05, rng.uniform(-0.2, 0.8, cfg.sizes()["n_pairs"]),
+                rng.uniform(-0.2, 0.9, m)) as p:
+        first = p.run(G, w, w, outputs=())
+        second = p.run(G, w, w, outputs=())
+        assert p.graph_launched()
+    for k in ("cost", "fcd_ks"):
+        np.testing.assert_array_equal(first[k], second[k])
