@@ -62,3 +62,15 @@ def test_predict_matches_forward_oracle(n_in, hidden, layers, out, n):
     # the oracle rounds where the device does: what is left is FP32 summation and rare BF16 rounding flips
     ref = mlp_oracle.loss_and_grads(m.get_params(), dims, X, np.zeros((n, out), np.float32))[2]
     assert np.linalg.norm(y - ref) <= 1e-3 * np.linalg.norm(ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_in,hidden,layers,out", [(19, 256, 4, 4), (3, 8, 1, 1), (17, 264, 2, 5), (33, 500, 2, 9)])
+def test_predict_rows_do_not_depend_on_the_call(n_in, hidden, layers, out):
+    """Large calls read the weights at their use, small ones copy them ahead: the same bits per row."""
+    m = S.MLP(n_in, out, hidden=hidden, layers=layers, max_batch=64, seed=1)
+    X = np.random.default_rng(hidden).standard_normal((5000, n_in)).astype(np.float32)
+    y = m.predict(X)
+    for n in (1, 16, 17, 333, 2368):
+        np.testing.assert_array_equal(m.predict(X[:n]), y[:n])
+        np.testing.assert_array_equal(m.predict(X[-n:]), y[-n:])
