@@ -2,7 +2,8 @@
 //
 // Same model and time loop as the reference's bnm kernel (bnm.cu:72-315) and
 // CPU path (bnm.cpp:167-290), re-laid out for Blackwell:
-//   * one CTA per particle (persistent over particles, two CTAs per SM); warp
+//   * one CTA per particle (persistent over particles, as many CTAs as an SM
+//     holds); warp
 //     w owns nodes 32w..32w+31.  The coupling G*J*(SC.S_E) is a register-
 //     blocked mat-vec: lane l = 4u+v of warp w keeps the 4 x KC block
 //     SC[32w+4u .. 32w+4u+3][KC v .. KC v+KC-1] in registers for the whole

@@ -106,7 +106,9 @@ extern "C" int bnm_gof_noalloc(const float* d_bold, int32_t n, int32_t frames, i
     const size_t o_fc = take((size_t)n * P * 4), o_wfc = take((size_t)n * W * P * 4);
     const size_t o_wsum = take((size_t)n * W * 2 * 8), o_hist = take((size_t)n * (m + 1) * 4);
     const size_t o_eq = take((size_t)n * (m + 1) * 4), o_nan = take((size_t)n * 4), o_zero = take(8 * (size_t)n + 8);
-    const size_t needed = off;
+    // (callers sized their batches by a layout with two P-int tables that the
+    // kernels no longer read: the limit stays where it was)
+    const size_t needed = off + 2 * align256((size_t)P * 4);
     if (needed > kScratchBytes) {
         char msg[256];
         std::snprintf(msg, sizeof msg,
