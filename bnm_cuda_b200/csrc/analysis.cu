@@ -321,23 +321,27 @@ __global__ void __launch_bounds__(256 + (RI + RJ + 1) / 2 * 32) fc_window_kernel
 
 // kTile x kTile outputs per CTA, RT x RT per thread (16 x 16 threads).  K
 // chunks are normalised (FP64) into one of two shared buffers while the other
-// is used, their loads in flight a chunk ahead.  Every output's sum runs over
-// K in order.  Few simulations with few windows leave most SMs without a
-// 64 x 64 tile (4 x 121 windows of 1122 pairs: 12 CTAs, 230 us with one buffer
-// and no load ahead), so those take 32 x 32 (40 CTAs, 54 us); many take the
-// larger tile, which reads each row half as often.
+// is used; their loads are in flight two chunks ahead.  Every output's sum runs
+// over K in order, so K cannot be split.  What bounds it: with few tiles the
+// chain of a chunk (load, conversion, barrier) on an SM with one CTA, with many
+// the shared-memory reads, which are four K at a time (rows of 36 floats: the
+// 16-byte reads of 8 rows touch all banks once).  Few simulations with few
+// windows leave most SMs without a 64 x 64 tile, so those take 32 x 32.
+// Measured with the window sums, one K per read -> now: 4 x 121 windows of
+// 1122 pairs (32 x 32) 56 -> 42 us, 2 x 136 of 39,800 1.48 -> 0.98 ms; 64 x 278
+// of 2450 (64 x 64) 1.20 -> 0.92 ms.
 constexpr int kTk = 32;
 
 template <int kTile>
-__global__ void __launch_bounds__(256) fcd_gram_kernel(FcdArgs a) {
+__global__ void __launch_bounds__(256, 2) fcd_gram_kernel(FcdArgs a) {
     constexpr int RT = kTile / 16, kLoads = kTile * kTk / 256;
     // blockIdx.x: lower-triangular tile index, blockIdx.y: simulation
     int t = blockIdx.x, ta = 0;
     while (t >= ta + 1) { t -= ta + 1; ta++; }
     const int tb = t;  // ta >= tb
     const int sim = blockIdx.y;
-    __shared__ float As[2][kTk][kTile + 1];
-    __shared__ float Bs[2][kTk][kTile + 1];
+    __shared__ __align__(16) float As[2][kTile][kTk + 4];
+    __shared__ __align__(16) float Bs[2][kTile][kTk + 4];
     __shared__ double mA[kTile], sA[kTile], mB[kTile], sB[kTile];
     const int a0 = ta * kTile, b0 = tb * kTile;
     const float* V = a.wfc + (size_t)sim * a.W * a.P;
@@ -359,23 +363,25 @@ __global__ void __launch_bounds__(256) fcd_gram_kernel(FcdArgs a) {
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
     const int lc = threadIdx.x % kTk, lr = threadIdx.x / kTk;  // column of this thread's loads, first row
     constexpr int kStep = 256 / kTk;
-    float va[kLoads], vb[kLoads];
-    auto fetch = [&](int k0) {
-        const int col = k0 + lc;
+    float v[2][2][kLoads];  // [chunk parity][A, B]
+    // no branch around a load or a conversion: the addresses are clamped, the
+    // values outside the rows and the pair range are replaced by zeros
+    auto fetch = [&](float (&v)[2][kLoads], int k0) {
+        const float* p = V + min(k0 + lc, a.p1 - 1);
 #pragma unroll
         for (int e = 0; e < kLoads; e++) {
-            const int ra = a0 + lr + e * kStep, rb = b0 + lr + e * kStep;
-            va[e] = ra < a.W && col < a.p1 ? V[(size_t)ra * a.P + col] : 0.f;
-            vb[e] = rb < a.W && col < a.p1 ? V[(size_t)rb * a.P + col] : 0.f;
+            v[0][e] = p[(size_t)min(a0 + lr + e * kStep, a.W - 1) * a.P];
+            v[1][e] = p[(size_t)min(b0 + lr + e * kStep, a.W - 1) * a.P];
         }
     };
-    auto store = [&](int buf, int k0) {  // centred and scaled; zero outside the rows and the pair range
-        const int col = k0 + lc;
+    auto store = [&](const float (&v)[2][kLoads], int buf, int k0) {  // centred and scaled
+        const bool in = k0 + lc < a.p1;
 #pragma unroll
         for (int e = 0; e < kLoads; e++) {
             const int r = lr + e * kStep;
-            As[buf][lc][r] = a0 + r < a.W && col < a.p1 ? (float)(((double)va[e] - mA[r]) * sA[r]) : 0.f;
-            Bs[buf][lc][r] = b0 + r < a.W && col < a.p1 ? (float)(((double)vb[e] - mB[r]) * sB[r]) : 0.f;
+            const float x = (float)(((double)v[0][e] - mA[r]) * sA[r]), y = (float)(((double)v[1][e] - mB[r]) * sB[r]);
+            As[buf][r][lc] = in && a0 + r < a.W ? x : 0.f;
+            Bs[buf][r][lc] = in && b0 + r < a.W ? y : 0.f;
         }
     };
     float acc[RT][RT];
@@ -383,26 +389,39 @@ __global__ void __launch_bounds__(256) fcd_gram_kernel(FcdArgs a) {
     for (int i = 0; i < RT; i++)
 #pragma unroll
         for (int j = 0; j < RT; j++) acc[i][j] = 0.f;
-    fetch(a.p0);
-    store(0, a.p0);
-    __syncthreads();
-    int buf = 0;
-    for (int k0 = a.p0; k0 < a.p1; k0 += kTk, buf ^= 1) {
-        const bool more = k0 + kTk < a.p1;
-        if (more) fetch(k0 + kTk);
-#pragma unroll 8
-        for (int c = 0; c < kTk; c++) {
-            float av[RT], bv[RT];
+    auto multiply = [&](int buf) {
+#pragma unroll 2
+        for (int c = 0; c < kTk; c += 4) {
+            float4 av[RT], bv[RT];
 #pragma unroll
-            for (int i = 0; i < RT; i++) av[i] = As[buf][c][ty * RT + i];
+            for (int i = 0; i < RT; i++) av[i] = *reinterpret_cast<const float4*>(&As[buf][ty * RT + i][c]);
 #pragma unroll
-            for (int j = 0; j < RT; j++) bv[j] = Bs[buf][c][tx + 16 * j];
+            for (int j = 0; j < RT; j++) bv[j] = *reinterpret_cast<const float4*>(&Bs[buf][tx + 16 * j][c]);
 #pragma unroll
             for (int i = 0; i < RT; i++)
 #pragma unroll
-                for (int j = 0; j < RT; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+                for (int j = 0; j < RT; j++) {
+                    acc[i][j] = fmaf(av[i].x, bv[j].x, acc[i][j]);
+                    acc[i][j] = fmaf(av[i].y, bv[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(av[i].z, bv[j].z, acc[i][j]);
+                    acc[i][j] = fmaf(av[i].w, bv[j].w, acc[i][j]);
+                }
         }
-        if (more) store(buf ^ 1, k0 + kTk);
+    };
+    fetch(v[0], a.p0);
+    fetch(v[1], a.p0 + kTk);
+    store(v[0], 0, a.p0);
+    __syncthreads();
+    for (int k0 = a.p0;;) {  // chunk k0 is in buffer 0, the next in v[1]
+        fetch(v[0], k0 + 2 * kTk);
+        multiply(0);
+        if ((k0 += kTk) >= a.p1) break;
+        store(v[1], 1, k0);
+        __syncthreads();
+        fetch(v[1], k0 + 2 * kTk);
+        multiply(1);
+        if ((k0 += kTk) >= a.p1) break;
+        store(v[0], 0, k0);
         __syncthreads();
     }
     bool any_nan = false;
@@ -647,8 +666,12 @@ cudaError_t bnm_launch_fcd(const FcdArgs& a, cudaStream_t st) {
         const int side = (a.W + tile - 1) / tile;
         return side * (side + 1) / 2;
     };
-    // the larger tile from two CTAs an SM on
-    if ((long long)tiles(64) * a.n_sims >= 296)
+    // The larger tile reads each row half as often and costs 2.5-2.8 of the
+    // smaller: it pays where there are two CTAs of it for each SM and the
+    // windows do not leave much of it empty (W = 278, 15 tiles against 45, 64
+    // simulations: 0.92 against 1.04 ms; W = 85, 3 against 6, 300 simulations:
+    // 132 against 110 us; 60 tiles in all: 169 against 116 us).
+    if ((long long)tiles(64) * a.n_sims >= 296 && 8 * tiles(64) < 3 * tiles(32))
         fcd_gram_kernel<64><<<dim3(tiles(64), a.n_sims), 256, 0, st>>>(a);
     else
         fcd_gram_kernel<32><<<dim3(tiles(32), a.n_sims), 256, 0, st>>>(a);
