@@ -511,6 +511,7 @@ __global__ void __launch_bounds__(1024) gof_kernel(GofArgs a) {
             for (int w = 0; w < 32; w++) t += wtot[w];
             total = t;
         }
+        __syncwarp();  // the cluster barrier is warp-wide (.aligned)
         cluster_sync();
         for (int r = 0; r < rank; r++) H += ld_cluster_u32(map_rank(smem_u32(&total), (uint32_t)r));
         const double invm = 1.0 / a.m, invn = 1.0 / a.n_fcd;
@@ -550,6 +551,7 @@ __global__ void __launch_bounds__(1024) gof_kernel(GofArgs a) {
         if (threadIdx.x == 0) st_cluster_f64(map_rank(smem_u32(&dks[rank]), 0), D);
     }
     // also keeps every CTA's total in place until all have read it
+    __syncwarp();
     cluster_sync();
     if (rank != 0) return;
     double D = 0.0;

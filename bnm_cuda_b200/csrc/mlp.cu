@@ -97,6 +97,11 @@ __device__ __forceinline__ uint32_t pack2(float x, float y) {
            ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(y)) << 16);
 }
 
+// The matrix instructions below are warp-wide (.aligned): all 32 lanes execute
+// them together.  A branch that only some lanes take (rows past the batch,
+// columns past a layer, Adam's plain expression) is followed by __syncwarp()
+// before the next of them.
+
 // 8 x 8 BF16 transpose across the warp: lane (g, t) holds row g, columns 2t, 2t + 1
 __device__ __forceinline__ uint32_t transpose8(uint32_t x) {
     uint32_t y;
@@ -139,6 +144,7 @@ template <int kFly, int nA, int nB, class F>
 __device__ __forceinline__ void mma_tiles(int kb, float (&d)[nA * nB][4], F load) {
 #pragma unroll
     for (int i = 0; i < nA * nB; i++) d[i][0] = d[i][1] = d[i][2] = d[i][3] = 0.f;
+    __syncwarp();
     int k0 = 0;
 #pragma unroll 1
     for (; k0 + kFly <= kb; k0 += kFly) mma_group<kFly, nA, nB>(k0, d, load);
@@ -233,6 +239,7 @@ __device__ __forceinline__ void gather_x(const Step& st, int step, int mb, int k
     uint4* x = st.lay[0].x + (step & 1 ? a.x0 : 0);
     uint2* xt = st.lay[0].xt + (step & 1 ? a.xt0 : 0) + lane;
     x[(size_t)(mb * kb + k) * 32 + lane] = make_uint4(v[0], v[1], v[2], v[3]);
+    __syncwarp();
     xt[(size_t)(2 * k * st.mt + mb) * 32] = make_uint2(transpose8(v[0]), transpose8(v[1]));
     xt[(size_t)((2 * k + 1) * st.mt + mb) * 32] = make_uint2(transpose8(v[2]), transpose8(v[3]));
 }
@@ -254,6 +261,7 @@ __device__ __forceinline__ void store_dz(const Step& st, const MlpLayer& z, int 
     // columns 8 nb .. are registers 0, 1 or 2, 3 of A block nb / 2
     reinterpret_cast<uint2*>(z.dzh + ((size_t)mb * (z.doutp / 16) + nb / 2) * 32 + lane)[nb & 1] = make_uint2(p0, p1);
     uint32_t* zt = reinterpret_cast<uint32_t*>(z.dzt + ((size_t)(nb / 2) * st.mt + mb) * 32 + lane) + (nb & 1);
+    __syncwarp();
     zt[0] = transpose8(p0);
     zt[2] = transpose8(p1);
 }
@@ -285,6 +293,7 @@ __device__ __forceinline__ void forward_tiles(const Step& st, int l, int mb, int
             const uint32_t p1 = m + 8 < B ? pack2(fmaxf(v[2], 0.f), fmaxf(v[3], 0.f)) : 0u;
             reinterpret_cast<uint2*>(z.x + ((size_t)(mb + i) * (z.dinp / 16) + nb / 2) * 32 + lane)[nb & 1] =
                 make_uint2(p0, p1);
+            __syncwarp();
             if (a.mode != kForward)
                 z.xt[((size_t)nb * st.mt + mb + i) * 32 + lane] = make_uint2(transpose8(p0), transpose8(p1));
             continue;
@@ -420,6 +429,7 @@ __device__ __forceinline__ void dw_task(const Step& st, int l, int task) {
 #pragma unroll
         for (int q = 0; q < 4; q++)
             if (!inside(i, q)) w[4 * i + q] = m[4 * i + q] = v[4 * i + q] = 0.f;  // the padding stays zero
+        __syncwarp();
         const size_t ei = e + (size_t)i * ot * 32;
         a.w[ei] = make_float4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
         a.m[ei] = make_float4(m[4 * i], m[4 * i + 1], m[4 * i + 2], m[4 * i + 3]);
@@ -460,6 +470,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) mlp_step_kernel(StepArgs args
                 f1(s1 + k);
             else
                 f2(s2 + k - (e1 - s1));
+            __syncwarp();
         }
         __syncwarp();
     };
@@ -650,6 +661,7 @@ __global__ void pack_kernel(const MlpLayer* layers, const float* flat, float4* w
             v[q] = o < y.dout && i < y.din ? flat[y.woff + (long long)o * y.din + i] : 0.f;
         }
         w[(size_t)(y.tile + k) * 32 + lane] = make_float4(v[0], v[1], v[2], v[3]);
+        __syncwarp();
         const uint32_t p0 = pack2(v[0], v[1]), p1 = pack2(v[2], v[3]);
         uint32_t* wp = reinterpret_cast<uint32_t*>(y.w + ((size_t)(2 * ob) * ki + ib / 2) * 32 + lane) + (ib & 1);
         wp[0] = p0;

@@ -1,0 +1,35 @@
+"""Training steps in which the lanes of a warp go different ways: gradients so
+small that some weights of a lane take Adam's plain expression, rows past the
+batch, layers whose last 32 outputs are not full (GPU)."""
+import numpy as np
+import pytest
+
+from bnm_cuda_b200 import surrogate as S
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_in,hidden,layers,out", [(19, 200, 2, 4), (5, 8, 1, 1), (37, 40, 3, 3), (16, 33, 2, 17)])
+def test_small_gradients_take_the_same_formula(n_in, hidden, layers, out):
+    from oracle import mlp_oracle
+
+    rng = np.random.default_rng(hidden)
+    X = rng.uniform(0.5, 1.5, (1, n_in)).astype(np.float32)
+    X[0, rng.permutation(n_in)[: n_in // 2]] *= np.float32(1e-13)  # squares of these gradients are below 1e-27
+    T = rng.standard_normal((1, out)).astype(np.float32)
+    m = S.MLP(n_in, out, hidden=hidden, layers=layers, max_batch=16, seed=5)
+    w = m.get_params()
+    loss, g = m.loss_and_grads(X, T)
+    dims = [n_in] + [hidden] * layers + [out]
+    ref = mlp_oracle.loss_and_grads(w, dims, X, T)[1]
+    first = slice(0, n_in * hidden)
+    for c in range(n_in):  # small columns too: products of one BF16 value each, a rounding flip is 2^-8
+        a, b = g[first].reshape(hidden, n_in)[:, c], ref[first].reshape(hidden, n_in)[:, c]
+        assert np.linalg.norm(a - b) <= 1e-2 * np.linalg.norm(b)
+    losses = m.fine_tune(X, T, epochs=1, batch=1, lr=1e-2, seed=0)
+    assert losses[0] == pytest.approx(loss, rel=1e-5)
+    # the first step from zero moments in FP32, every operation rounded to nearest
+    f = np.float32
+    b1, b2 = f(0.9), f(0.999)
+    mm, v = (f(1) - b1) * g, (f(1) - b2) * g * g
+    want = w - f(1e-2) * (mm / (f(1) - b1)) / (np.sqrt(v / (f(1) - b2)) + f(1e-8))
+    np.testing.assert_array_equal(m.get_params(), want)
