@@ -130,14 +130,10 @@ __device__ __forceinline__ R dot_smem(const Vec<R>* sc, int nodes, const R* S, i
     return c;
 }
 
-// Threads of the kernel for N nodes, and whether the populations have warps
-// of their own: up to 256 nodes, where two threads a node leave each thread
-// 128 registers.
-__host__ __device__ inline bool generic_split(int N) { return N <= 256; }
-
-// Dynamic shared memory: S_E[2][npad], S_I[2][npad] (+ SC[cols / n][N] Vecs when kSmem).
-template <typename R, bool kSplit, bool kSmem>
-__global__ void __launch_bounds__(kSplit ? 512 : sizeof(R) == 8 ? 640 : 1024) integrate_generic_kernel(SimArgs a) {
+// Dynamic shared memory: S_E[2][npad], S_I[2][npad] (+ SC[cols / n][N] Vecs when
+// kSmem).  kSplit: two threads a node, kThreads the largest CTA.
+template <typename R, bool kSplit, bool kSmem, int kThreads>
+__global__ void __launch_bounds__(kThreads) integrate_generic_kernel(SimArgs a) {
     typedef Model<R> C;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int N = a.N, npad = kSplit ? blockDim.x / 2 : blockDim.x;
@@ -342,28 +338,33 @@ __global__ void __launch_bounds__(kSplit ? 512 : sizeof(R) == 8 ? 640 : 1024) in
     }
 }
 
-// Threads, shared memory and launch for a.N nodes; SC goes to shared memory
-// where it fits an SM (FP64 up to 164 nodes, FP32 up to 233).
-template <typename R, bool kSplit, bool kSmem>
+template <typename R, bool kSplit, bool kSmem, int kThreads>
 static cudaError_t launch_generic_t(const SimArgs& a, int threads, size_t smem, int num_sms, cudaStream_t st) {
-    auto* fn = integrate_generic_kernel<R, kSplit, kSmem>;
+    auto* fn = integrate_generic_kernel<R, kSplit, kSmem, kThreads>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int grid = a.n_sims < 2 * num_sms ? a.n_sims : 2 * num_sms;
     fn<<<grid, threads, smem, st>>>(a);
     return cudaGetLastError();
 }
+// The variant for N nodes and n particles:
+//   SC in shared memory where it fits an SM (FP64 up to 164 nodes, FP32 up to
+//   234), two threads a node;
+//   else SC rows from global memory, two threads a node up to 256 nodes;
+//   else one thread a node: FP64 with 96 registers while the CTA leaves each
+//   thread that many (640 threads), above with 64 and some spills.
 template <typename R>
 static cudaError_t launch_generic(const SimArgs& a, int num_sms, cudaStream_t st) {
     const int npad = ((a.N + 31) / 32) * 32;
     if (npad > 1024) return cudaErrorInvalidValue;
-    const bool split = generic_split(a.N);
-    const int threads = split ? 2 * npad : npad;
     const size_t smem = 4 * (size_t)npad * sizeof(R);
     const size_t sc_bytes = (size_t)a.N * ((a.N + kColPad - 1) / kColPad * kColPad) * sizeof(R);
-    if (!split) return launch_generic_t<R, false, false>(a, threads, smem, num_sms, st);  // SC never fits
-    if (smem + sc_bytes > 220 * 1024) return launch_generic_t<R, true, false>(a, threads, smem, num_sms, st);
-    return launch_generic_t<R, true, true>(a, threads, smem + sc_bytes, num_sms, st);
+    if (smem + sc_bytes <= 220 * 1024)
+        return launch_generic_t<R, true, true, 512>(a, 2 * npad, smem + sc_bytes, num_sms, st);
+    if (npad <= 256) return launch_generic_t<R, true, false, 512>(a, 2 * npad, smem, num_sms, st);
+    if constexpr (sizeof(R) == 8)
+        if (npad <= 640) return launch_generic_t<R, false, false, 640>(a, npad, smem, num_sms, st);
+    return launch_generic_t<R, false, false, 1024>(a, npad, smem, num_sms, st);
 }
 
 }  // namespace BNM_GENERIC_NS
