@@ -52,7 +52,7 @@ struct SimArgs {
     int noise_ld;          // node stride of the noise table (N, or N + 1 when padded for an odd N)
     int n_real;            // nodes of the simulation; the kernel's N may add one padding node
     const float* sc_f32;   // [N][sc_ld] row-major, zero padded
-    const double* sc_f64;  // [N][N]
+    const double* sc_f64;  // [N][N], transposed: element (i, k) at k N + i
     int sc_ld;
     // outputs
     float* bold;        // [n][frames][N] (fp32 kernels)

@@ -63,12 +63,13 @@ __device__ __forceinline__ void store_bold<float>(const SimArgs& a, size_t idx, 
 template <>
 __device__ __forceinline__ void store_bold<double>(const SimArgs& a, size_t idx, double v) { a.bold_f64[idx] = v; }
 
-// Coupling of one node, the products added in column order, SC rows in global
-// memory.
+// Coupling of one node, the products added in column order, SC in global
+// memory, its columns `step` values apart.
 template <typename R>
-__device__ __forceinline__ R dot_row(const R* sc, const R* S, int N) {
+__device__ __forceinline__ R dot_global(const R* sc, int step, const R* S, int N) {
     R c = 0;
-    for (int k = 0; k < N; k++) c += sc[k] * S[k];
+#pragma unroll 8
+    for (int k = 0; k < N; k++) c += sc[(size_t)k * step] * S[k];
     return c;
 }
 
@@ -137,7 +138,8 @@ __global__ void __launch_bounds__(kThreads) integrate_generic_kernel(SimArgs a) 
     typedef Model<R> C;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int N = a.N, npad = kSplit ? blockDim.x / 2 : blockDim.x;
-    const int ld = (sizeof(R) == 4) ? a.sc_ld : N;
+    // SC in global memory: FP32 by rows (shared with the other integrators), FP64 by columns
+    const int row = sizeof(R) == 4 ? a.sc_ld : 1, step = sizeof(R) == 4 ? 1 : N;
     R* S_buf = reinterpret_cast<R*>(smem_raw);
     R* I_buf = S_buf + 2 * npad;
     const R* SC = sc_ptr<R>(a);
@@ -146,8 +148,9 @@ __global__ void __launch_bounds__(kThreads) integrate_generic_kernel(SimArgs a) 
         constexpr int V = Vec<R>::n;
         R* sc_s = I_buf + 2 * npad;
         for (int i = threadIdx.x; i < N * cols; i += blockDim.x) {
-            const int r = i / cols, c = i - r * cols;
-            sc_s[((c / V) * N + r) * V + c % V] = c < N ? SC[(size_t)r * ld + c] : (R)0;
+            // consecutive threads take what is consecutive in global memory
+            const int r = sizeof(R) == 4 ? i / cols : i % N, c = sizeof(R) == 4 ? i % cols : i / N;
+            sc_s[((c / V) * N + r) * V + c % V] = c < N ? SC[(size_t)r * row + (size_t)c * step] : (R)0;
         }
         SC = sc_s;
     }
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(kThreads) integrate_generic_kernel(SimArgs a) 
     const bool isE = !kSplit || (int)threadIdx.x < npad, isI = !kSplit || !isE;
     const int j = kSplit && !isE ? threadIdx.x - npad : threadIdx.x;
     const bool act = j < N;
-    const R* sc_row = SC + (size_t)(act ? j : 0) * (kSmem ? Vec<R>::n : ld);
+    const R* sc_row = SC + (size_t)(act ? j : 0) * (kSmem ? Vec<R>::n : row);
     const unsigned int duration = a.samp_end - a.samp_start + 1;
     const size_t plane = (size_t)a.noise_ld;  // node stride of the noise table
     // noise of this thread's node: both values, or its own population's
@@ -227,7 +230,7 @@ __global__ void __launch_bounds__(kThreads) integrate_generic_kernel(SimArgs a) 
                         if constexpr (kSmem)
                             coupling = dot_smem<R>(reinterpret_cast<const Vec<R>*>(sc_row), N, Sp, cols);
                         else
-                            coupling = dot_row<R>(sc_row, Sp, N);
+                            coupling = dot_global<R>(sc_row, step, Sp, N);
                         IE = base + coupling * G * C::J_NMDA - inh;
                         R eE = dexp(-C::d_E * (C::a_E * IE - C::b_E));
                         rE = (C::a_E * IE - C::b_E) / (1 - eE);
@@ -350,7 +353,12 @@ static cudaError_t launch_generic_t(const SimArgs& a, int threads, size_t smem, 
 // The variant for N nodes and n particles:
 //   SC in shared memory where it fits an SM (FP64 up to 164 nodes, FP32 up to
 //   234), two threads a node;
-//   else SC rows from global memory, two threads a node up to 256 nodes;
+//   else SC from global memory, two threads a node up to 256 nodes.  In FP64
+//   that takes 122 registers a thread and an SM holds one CTA, where it held
+//   two with one thread a node; with SC by rows, a cache line per lane, that
+//   cost calls of more particles than SMs (N = 200, 296 particles of 600 ms: 176
+//   ms with one thread a node, 193 with two).  By columns the L1 no longer
+//   bounds it: 81 ms, and 40 with 148 particles (103 and 96 by rows);
 //   else one thread a node: FP64 with 96 registers while the CTA leaves each
 //   thread that many (640 threads), above with 64 and some spills.
 template <typename R>
