@@ -469,6 +469,43 @@ static int d2h(T* host, const T* dev, size_t n, cudaStream_t st) {
     return BNM_OK;
 }
 
+// Pieces of a transfer of `rows` rows of `len` values, `pitch` values apart on
+// the device and contiguous on the host: whole rows, or parts of one row that
+// is longer than a piece.  Piece k: offsets on the host and the device, rows and
+// values per row.  A piece of one row, or of rows that follow one another, is
+// one contiguous copy; others are 2-D copies, whose pitch in bytes CUDA limits
+// to 2^31 - 1 -- beyond that a piece is a single row.
+struct IoPieces {
+    size_t rows, len, pitch, group, parts, count;
+    IoPieces(size_t r, size_t l, size_t p) : rows(r), len(l), pitch(p) {
+        const bool far = pitch * 4 > 0x7fffffff && pitch != len;
+        group = far ? 1 : std::max<size_t>(1, kIoPiece / len);
+        parts = (len + kIoPiece - 1) / kIoPiece;
+        count = parts > 1 ? rows * parts : (rows + group - 1) / group;
+    }
+    void at(size_t k, size_t& host, size_t& dev, size_t& r, size_t& l) const {
+        const size_t row = parts > 1 ? k / parts : k * group, col = parts > 1 ? k % parts * kIoPiece : 0;
+        host = row * len + col;
+        dev = row * pitch + col;
+        r = parts > 1 ? 1 : std::min(group, rows - row);
+        l = parts > 1 ? std::min(kIoPiece, len - col) : len;
+    }
+    bool contiguous(size_t r) const { return r == 1 || pitch == len; }
+};
+
+// Piece k of a transfer for tests: host and device offset, rows, values per
+// row, contiguous or not; returns the number of pieces.
+extern "C" int64_t bnm_transfer_piece(int64_t rows, int64_t len, int64_t pitch, int64_t k, int64_t* out5) {
+    const IoPieces ps(rows, len, pitch);
+    if (k >= 0 && (size_t)k < ps.count) {
+        size_t h, d, r, l;
+        ps.at(k, h, d, r, l);
+        const int64_t v[5] = {(int64_t)h, (int64_t)d, (int64_t)r, (int64_t)l, ps.contiguous(r)};
+        std::copy(v, v + 5, out5);
+    }
+    return (int64_t)ps.count;
+}
+
 // `rows` rows of `len` values between the caller's doubles (contiguous) and the
 // device's floats (rows `pitch` values apart), converted on the way; upload or
 // download, on the plan's stream.  A download is complete on return; an upload
@@ -479,15 +516,24 @@ static int transfer_f32(bnm_plan* p, bool up, double* host, float* dev, size_t r
     const size_t total = rows * len;
     if (!host || !total) return BNM_OK;
     cudaStream_t st = p->st;
-    const cudaMemcpyKind kind = up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+    const IoPieces pieces(rows, len, pitch);
+    // r rows of l values between h (contiguous) and d
+    auto move = [&](float* h, float* d, size_t r, size_t l) {
+        if (pieces.contiguous(r))
+            return up ? cudaMemcpyAsync(d, h, r * l * 4, cudaMemcpyHostToDevice, st)
+                      : cudaMemcpyAsync(h, d, r * l * 4, cudaMemcpyDeviceToHost, st);
+        return up ? cudaMemcpy2DAsync(d, pitch * 4, h, l * 4, l * 4, r, cudaMemcpyHostToDevice, st)
+                  : cudaMemcpy2DAsync(h, l * 4, d, pitch * 4, l * 4, r, cudaMemcpyDeviceToHost, st);
+    };
     if (total < kIoSmall) {
         std::vector<float> tmp(total);
         if (up)
             for (size_t i = 0; i < total; i++) tmp[i] = (float)host[i];
-        if (up)
-            BNM_CUDA_TRY(cudaMemcpy2DAsync(dev, pitch * 4, tmp.data(), len * 4, len * 4, rows, kind, st));
-        else
-            BNM_CUDA_TRY(cudaMemcpy2DAsync(tmp.data(), len * 4, dev, pitch * 4, len * 4, rows, kind, st));
+        for (size_t k = 0; k < pieces.count; k++) {
+            size_t h, d, r, l;
+            pieces.at(k, h, d, r, l);
+            BNM_CUDA_TRY(move(tmp.data() + h, dev + d, r, l));
+        }
         BNM_CUDA_TRY(cudaStreamSynchronize(st));
         if (!up)
             for (size_t i = 0; i < total; i++) host[i] = tmp[i];
@@ -497,45 +543,24 @@ static int transfer_f32(bnm_plan* p, bool up, double* host, float* dev, size_t r
         for (auto& e : p->io_ev) BNM_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         BNM_CUDA_TRY(cudaMallocHost((void**)&p->io_slots, 2 * kIoThreads * kIoPiece * 4));
     }
-    // pieces: whole rows, or parts of one row that is longer than a piece
-    const size_t group = std::max<size_t>(1, kIoPiece / len), parts = (len + kIoPiece - 1) / kIoPiece;
-    const size_t n_pieces = parts > 1 ? rows * parts : (rows + group - 1) / group;
     std::atomic<int> error{(int)cudaSuccess};
-    auto piece = [&](size_t k, size_t& off, size_t& n_rows, size_t& n_len, float*& d) {
-        if (parts > 1) {
-            const size_t r = k / parts, c = k % parts * kIoPiece;
-            off = r * len + c;
-            n_rows = 1;
-            n_len = std::min(kIoPiece, len - c);
-            d = dev + r * pitch + c;
-        } else {
-            off = k * group * len;
-            n_rows = std::min(group, rows - k * group);
-            n_len = len;
-            d = dev + k * group * pitch;
-        }
-    };
     auto work = [&](int t, int n_threads) {
-        size_t off, r, l;
-        float* d;
+        size_t off, d, r, l;
         cudaError_t e = cudaSetDevice(p->cfg.device);
         auto copy = [&](size_t k, int slot) {  // enqueue piece k through a slot
-            piece(k, off, r, l, d);
-            float* h = p->io_slots + (size_t)slot * kIoPiece;
-            if (e == cudaSuccess)
-                e = up ? cudaMemcpy2DAsync(d, pitch * 4, h, l * 4, l * 4, r, kind, st)
-                       : cudaMemcpy2DAsync(h, l * 4, d, pitch * 4, l * 4, r, kind, st);
+            pieces.at(k, off, d, r, l);
+            if (e == cudaSuccess) e = move(p->io_slots + (size_t)slot * kIoPiece, dev + d, r, l);
             if (e == cudaSuccess) e = cudaEventRecord(p->io_ev[slot], st);
         };
         int turn = 0;
-        if (!up && (size_t)t < n_pieces) copy(t, 2 * t);
-        for (size_t k = t; k < n_pieces && e == cudaSuccess; k += n_threads, turn ^= 1) {
+        if (!up && (size_t)t < pieces.count) copy(t, 2 * t);
+        for (size_t k = t; k < pieces.count && e == cudaSuccess; k += n_threads, turn ^= 1) {
             const int slot = 2 * t + turn;
             const float* h = p->io_slots + (size_t)slot * kIoPiece;
-            if (!up && k + n_threads < n_pieces) copy(k + n_threads, slot ^ 1);
+            if (!up && k + n_threads < pieces.count) copy(k + n_threads, slot ^ 1);
             if (e == cudaSuccess) e = cudaEventSynchronize(p->io_ev[slot]);  // the slot's last copy
             if (e != cudaSuccess) break;
-            piece(k, off, r, l, d);
+            pieces.at(k, off, d, r, l);
             if (up) {
                 float* w = p->io_slots + (size_t)slot * kIoPiece;
                 const double* src = host + off;
@@ -548,7 +573,7 @@ static int transfer_f32(bnm_plan* p, bool up, double* host, float* dev, size_t r
         }
         if (e != cudaSuccess) error = (int)e;
     };
-    int n_threads = total < kIoParallel ? 1 : (int)std::min<size_t>(kIoThreads, n_pieces);
+    int n_threads = total < kIoParallel ? 1 : (int)std::min<size_t>(kIoThreads, pieces.count);
     const unsigned cores = std::thread::hardware_concurrency();
     if (cores) n_threads = std::min(n_threads, (int)cores);
     std::thread th[kIoThreads];
