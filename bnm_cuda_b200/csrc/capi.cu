@@ -138,6 +138,10 @@ constexpr int kIoThreads = 4;
 constexpr size_t kIoPiece = 128 * 1024;    // values: 512 KB
 constexpr size_t kIoSmall = 64 * 1024;     // below: one pageable copy
 constexpr size_t kIoParallel = 256 * 1024; // below: the calling thread alone
+// A plan page-locks slots only for the threads that a transfer of its own has
+// used: locking and releasing memory costs a program that makes a plan for one
+// call (4 x 300 frames x 60 nodes, first check_fit_bold of a plan: 2.9 ms with
+// the slots of all four threads, 1.1 with those of one).
 
 constexpr int kPlaceWs = 2 + 256;  // placement claim word + CTAs per SM
 
@@ -199,8 +203,9 @@ struct bnm_plan {
     std::vector<float> hist_x;  // G, mean wEE, mean wEI per simulated particle
     std::vector<int> hist_tr;
     size_t hist_next = 0;
-    // page-locked slots of transfer_f32 (allocated on first use) and the last copy from or to each
-    float* io_slots = nullptr;
+    // page-locked slots of transfer_f32, two per thread (for as many threads as a transfer has
+    // used; io_mem: the allocations), and the last copy from or to each
+    float *io_slots[kIoThreads] = {}, *io_mem[kIoThreads] = {};
     cudaEvent_t io_ev[2 * kIoThreads] = {};
     double timings[6] = {0, 0, 0, 0, 0, 0};
     // tensor-core Gram kernels alone: one event pair per launch (FC, then each FCD chunk)
@@ -226,7 +231,8 @@ extern "C" void bnm_plan_destroy(bnm_plan* p) {
     if (p->run_graph) cudaGraphDestroy(p->run_graph);
     if (p->pinned) cudaFreeHost(p->pinned);
     if (p->io_order) cudaFreeHost(p->io_order);
-    if (p->io_slots) cudaFreeHost(p->io_slots);
+    for (auto& h : p->io_mem)
+        if (h) cudaFreeHost(h);
     for (auto& e : p->io_ev)
         if (e) cudaEventDestroy(e);
     for (auto& e : p->ev)
@@ -525,7 +531,25 @@ static int transfer_f32(bnm_plan* p, bool up, double* host, float* dev, size_t r
         return up ? cudaMemcpy2DAsync(d, pitch * 4, h, l * 4, l * 4, r, cudaMemcpyHostToDevice, st)
                   : cudaMemcpy2DAsync(h, l * 4, d, pitch * 4, l * 4, r, cudaMemcpyDeviceToHost, st);
     };
-    if (total < kIoSmall) {
+    // the threads that the transfer is worth and for which there are slots
+    int n_threads = total < kIoSmall ? 0 : total < kIoParallel ? 1 : (int)std::min<size_t>(kIoThreads, pieces.count);
+    const unsigned cores = std::thread::hardware_concurrency();
+    if (cores) n_threads = std::min(n_threads, (int)cores);
+    int have = 0;
+    while (have < n_threads && p->io_slots[have]) have++;
+    if (have < n_threads) {  // slots of the threads that have none, in one piece
+        for (int k = 2 * have; k < 2 * n_threads; k++)
+            if (!p->io_ev[k]) BNM_CUDA_TRY(cudaEventCreateWithFlags(&p->io_ev[k], cudaEventDisableTiming));
+        float*& mem = p->io_mem[have];
+        if (cudaMallocHost((void**)&mem, (size_t)(n_threads - have) * 2 * kIoPiece * 4) == cudaSuccess) {
+            for (int t = have; t < n_threads; t++) p->io_slots[t] = mem + (size_t)(t - have) * 2 * kIoPiece;
+        } else {
+            cudaGetLastError();
+            mem = nullptr;
+            n_threads = have;
+        }
+    }
+    if (!n_threads) {  // a small transfer, or no page-locked memory to be had: through a pageable array
         std::vector<float> tmp(total);
         if (up)
             for (size_t i = 0; i < total; i++) tmp[i] = (float)host[i];
@@ -539,30 +563,27 @@ static int transfer_f32(bnm_plan* p, bool up, double* host, float* dev, size_t r
             for (size_t i = 0; i < total; i++) host[i] = tmp[i];
         return BNM_OK;
     }
-    if (!p->io_slots) {
-        for (auto& e : p->io_ev) BNM_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        BNM_CUDA_TRY(cudaMallocHost((void**)&p->io_slots, 2 * kIoThreads * kIoPiece * 4));
-    }
     std::atomic<int> error{(int)cudaSuccess};
+    auto slot_ptr = [&](int slot) { return p->io_slots[slot / 2] + (size_t)(slot & 1) * kIoPiece; };
     auto work = [&](int t, int n_threads) {
         size_t off, d, r, l;
         cudaError_t e = cudaSetDevice(p->cfg.device);
         auto copy = [&](size_t k, int slot) {  // enqueue piece k through a slot
             pieces.at(k, off, d, r, l);
-            if (e == cudaSuccess) e = move(p->io_slots + (size_t)slot * kIoPiece, dev + d, r, l);
+            if (e == cudaSuccess) e = move(slot_ptr(slot), dev + d, r, l);
             if (e == cudaSuccess) e = cudaEventRecord(p->io_ev[slot], st);
         };
         int turn = 0;
         if (!up && (size_t)t < pieces.count) copy(t, 2 * t);
         for (size_t k = t; k < pieces.count && e == cudaSuccess; k += n_threads, turn ^= 1) {
             const int slot = 2 * t + turn;
-            const float* h = p->io_slots + (size_t)slot * kIoPiece;
+            const float* h = slot_ptr(slot);
             if (!up && k + n_threads < pieces.count) copy(k + n_threads, slot ^ 1);
             if (e == cudaSuccess) e = cudaEventSynchronize(p->io_ev[slot]);  // the slot's last copy
             if (e != cudaSuccess) break;
             pieces.at(k, off, d, r, l);
             if (up) {
-                float* w = p->io_slots + (size_t)slot * kIoPiece;
+                float* w = slot_ptr(slot);
                 const double* src = host + off;
                 for (size_t i = 0; i < r * l; i++) w[i] = (float)src[i];
                 copy(k, slot);
@@ -573,9 +594,6 @@ static int transfer_f32(bnm_plan* p, bool up, double* host, float* dev, size_t r
         }
         if (e != cudaSuccess) error = (int)e;
     };
-    int n_threads = total < kIoParallel ? 1 : (int)std::min<size_t>(kIoThreads, pieces.count);
-    const unsigned cores = std::thread::hardware_concurrency();
-    if (cores) n_threads = std::min(n_threads, (int)cores);
     std::thread th[kIoThreads];
     int started = 1;  // thread 0 is the caller
     try {
