@@ -461,19 +461,26 @@ __global__ void __launch_bounds__(kStepThreads, 1) mlp_step_kernel(StepArgs args
     const int mt = (B + 15) / 16, mg = (mt + 1) / 2;  // blocks of 16 rows, taken in twos
     Step st{args, lay, 0, make_float2(1.f, 1.f), 1.0, 1.0, mt};
 
-    // this CTA's shares of two task lists, dealt to its warps
-    auto for_tasks = [&](int n1, int n2, auto&& f1, auto&& f2) {
-        const int p1 = (n1 + nc - 1) / nc, p2 = (n2 + nc - 1) / nc;
-        const int s1 = min(n1, c * p1), e1 = min(n1, s1 + p1), s2 = min(n2, c * p2), e2 = min(n2, s2 + p2);
-        for (int k = warp; k < (e1 - s1) + (e2 - s2); k += kStepWarps) {
-            if (k < e1 - s1)
+    // this CTA's shares of up to three task lists, dealt to its warps.  Every
+    // list is shared out by itself: as one, gathers and weight tiles of the last
+    // phase fell to different CTAs, and with many inputs one CTA had all tiles
+    // (4096 inputs, 256 wide, batch 4096: 11.5 ms a step, now 1.9)
+    auto for_tasks = [&](int n1, int n2, int n3, auto&& f1, auto&& f2, auto&& f3) {
+        const int p1 = (n1 + nc - 1) / nc, p2 = (n2 + nc - 1) / nc, p3 = (n3 + nc - 1) / nc;
+        const int s1 = min(n1, c * p1), s2 = min(n2, c * p2), s3 = min(n3, c * p3);
+        const int l1 = min(n1, s1 + p1) - s1, l2 = l1 + min(n2, s2 + p2) - s2, l3 = l2 + min(n3, s3 + p3) - s3;
+        for (int k = warp; k < l3; k += kStepWarps) {
+            if (k < l1)
                 f1(s1 + k);
+            else if (k < l2)
+                f2(s2 + k - l1);
             else
-                f2(s2 + k - (e1 - s1));
+                f3(s3 + k - l2);
             __syncwarp();
         }
         __syncwarp();
     };
+    auto none = [](int) {};
     auto dw_tasks = [&](int l) { return (lay[l].doutp / 16) * (lay[l].dinp / 16) + (lay[l].dout + 31) / 32; };
 
     // gather tasks of a step: operand blocks, then targets
@@ -484,7 +491,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) mlp_step_kernel(StepArgs args
         else
             gather_t(args, step, task - nx);
     };
-    for_tasks(nx + nt, 0, [&](int task) { gather(0, task); }, [](int) {});
+    for_tasks(nx + nt, 0, 0, [&](int task) { gather(0, task); }, none, none);
     cluster_sync();
 
     for (int step = 0; step < args.steps; step++) {
@@ -496,13 +503,13 @@ __global__ void __launch_bounds__(kStepThreads, 1) mlp_step_kernel(StepArgs args
         }
 
         for (int l = 0; l < L; l++) {
-            for_tasks(mg * (lay[l].doutp / 8), 0, [&](int task) {
+            for_tasks(mg * (lay[l].doutp / 8), 0, 0, [&](int task) {
                 const int mb = 2 * (task % mg), nb = task / mg;
                 if (mb + 1 < mt)
                     forward_tiles<2>(st, l, mb, nb);
                 else
                     forward_tiles<1>(st, l, mb, nb);
-            }, [](int) {});
+            }, none, none);
             cluster_sync();
         }
         if (args.mode == kForward) continue;
@@ -525,23 +532,18 @@ __global__ void __launch_bounds__(kStepThreads, 1) mlp_step_kernel(StepArgs args
             if (threadIdx.x == 0) args.loss[step] = red[0] / (float)(B * args.out);
         }
         for (int l = L - 1; l >= 1; l--) {
-            for_tasks(mg * (lay[l].dinp / 8), l < L - 1 ? dw_tasks(l + 1) : 0, [&](int task) {
+            for_tasks(mg * (lay[l].dinp / 8), l < L - 1 ? dw_tasks(l + 1) : 0, 0, [&](int task) {
                 const int mb = 2 * (task % mg), nb = task / mg;
                 if (mb + 1 < mt)
                     dx_tiles<2>(st, l, mb, nb);
                 else
                     dx_tiles<1>(st, l, mb, nb);
-            }, [&](int task) { dw_task(st, l + 1, task); });
+            }, [&](int task) { dw_task(st, l + 1, task); }, none);
             cluster_sync();
         }
         // the last phase also gathers the next step's rows
-        const int n0 = dw_tasks(0), ng = step + 1 < args.steps ? nx + nt : 0;
-        for_tasks(dw_tasks(1), n0 + ng, [&](int task) { dw_task(st, 1, task); }, [&](int task) {
-            if (task < ng)
-                gather(step + 1, task);
-            else
-                dw_task(st, 0, task - ng);
-        });
+        for_tasks(dw_tasks(1), step + 1 < args.steps ? nx + nt : 0, dw_tasks(0), [&](int task) { dw_task(st, 1, task); },
+                  [&](int task) { gather(step + 1, task); }, [&](int task) { dw_task(st, 0, task); });
         cluster_sync();
     }
 }
