@@ -443,7 +443,10 @@ __device__ __forceinline__ void dw_task(const Step& st, int l, int task) {
 }
 
 // One cluster; CTA c of it takes the c-th share of a phase's tiles, a warp per
-// tile.  Phases of a step, each ending in a cluster barrier:
+// tile.  A forward pass alone may have several clusters: they take blocks of
+// rows of their own, and none waits for another (one cluster for all rows took
+// 26 ms for 8192 rows of 19-3x4096-4 where a launch per GEMM had taken 22; now
+// 7.7).  Phases of a step, each ending in a cluster barrier:
 //   forward of layer 0 .. L-1 (the last also forms the output gradient);
 //   for l = L-1 .. 1: dX of layer l, with dW / db (and Adam) of layer l + 1;
 //   dW / db of layers 1 and 0, and the next step's rows of X and T.
@@ -458,7 +461,10 @@ __global__ void __launch_bounds__(kStepThreads, 1) mlp_step_kernel(StepArgs args
             reinterpret_cast<uint32_t*>(s_lay)[e] = reinterpret_cast<const uint32_t*>(args.layers)[e];
     __syncthreads();
     const MlpLayer* lay = L <= kSmemLayers ? s_lay : args.layers;
-    const int mt = (B + 15) / 16, mg = (mt + 1) / 2;  // blocks of 16 rows, taken in twos
+    // blocks of 16 rows, taken in twos; this cluster's: mg twos from block mb0
+    const int mt = (B + 15) / 16, twos = (mt + 1) / 2;
+    const int clusters = gridDim.x / nc, per = (twos + clusters - 1) / clusters;
+    const int mb0 = 2 * min(twos, (int)(blockIdx.x / nc) * per), mg = min(twos, mb0 / 2 + per) - mb0 / 2;
     Step st{args, lay, 0, make_float2(1.f, 1.f), 1.0, 1.0, mt};
 
     // this CTA's shares of up to three task lists, dealt to its warps.  Every
@@ -484,10 +490,10 @@ __global__ void __launch_bounds__(kStepThreads, 1) mlp_step_kernel(StepArgs args
     auto dw_tasks = [&](int l) { return (lay[l].doutp / 16) * (lay[l].dinp / 16) + (lay[l].dout + 31) / 32; };
 
     // gather tasks of a step: operand blocks, then targets
-    const int kx = lay[0].dinp / 16, nx = mt * kx, nt = args.mode == kForward ? 0 : (B * args.out + 31) / 32;
+    const int kx = lay[0].dinp / 16, nx = (min(mt, mb0 + 2 * mg) - min(mt, mb0)) * kx, nt = args.mode == kForward ? 0 : (B * args.out + 31) / 32;
     auto gather = [&](int step, int task) {
         if (task < nx)
-            gather_x(st, step, task / kx, task % kx);
+            gather_x(st, step, mb0 + task / kx, task % kx);
         else
             gather_t(args, step, task - nx);
     };
@@ -504,7 +510,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) mlp_step_kernel(StepArgs args
 
         for (int l = 0; l < L; l++) {
             for_tasks(mg * (lay[l].doutp / 8), 0, 0, [&](int task) {
-                const int mb = 2 * (task % mg), nb = task / mg;
+                const int mb = mb0 + 2 * (task % mg), nb = task / mg;
                 if (mb + 1 < mt)
                     forward_tiles<2>(st, l, mb, nb);
                 else
@@ -701,7 +707,8 @@ struct bnm_mlp {
     std::vector<MlpLayer> lay;
     MlpLayer* d_lay = nullptr;
     long long n_params = 0;
-    int cluster = 8;        // CTAs of mlp_step_kernel
+    int cluster = 8;        // CTAs of a cluster of mlp_step_kernel
+    int fwd_clusters = 1;   // clusters of a forward pass: as many as the SMs would hold
     int width = 0;          // widest padded layer input
     size_t pred_smem = 0;   // shared memory of mlp_predict_kernel, 0: too wide for it
     size_t ahead_smem = 0;  // ... with the weights copied ahead, 0: too wide
@@ -797,6 +804,8 @@ static int mlp_init(bnm_mlp* p, uint64_t seed) {
     // predict: rows travel through a page-locked buffer of at most 16 MiB (or max_batch rows)
     const size_t row_bytes = (size_t)(p->in + p->out) * 4;
     p->pred_rows = (int)std::max<size_t>(p->max_batch, std::min<size_t>(8192, ((size_t)16 << 20) / row_bytes));
+    int sms = 0;
+    BNM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device));
     p->pred_smem = (size_t)2 * 16 * p->width * 2;
     if (p->pred_smem > 200 * 1024) p->pred_smem = 0;
     if (p->pred_smem) {
@@ -804,8 +813,6 @@ static int mlp_init(bnm_mlp* p, uint64_t seed) {
                                           200 * 1024));
         const size_t ahead = p->pred_smem + (size_t)kPredWarps * kPredDepth * p->width * 2 * sizeof(uint2);
         if (ahead <= 210 * 1024) {
-            int sms = 0;
-            BNM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device));
             BNM_CUDA_TRY(cudaFuncSetAttribute(mlp_predict_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               210 * 1024));
             p->ahead_smem = ahead;
@@ -828,6 +835,7 @@ static int mlp_init(bnm_mlp* p, uint64_t seed) {
     if (cudaOccupancyMaxActiveClusters(&clusters, mlp_step_kernel, &cfg) == cudaSuccess && clusters > 0)
         p->cluster = 16;
     cudaGetLastError();
+    p->fwd_clusters = std::max(1, sms / p->cluster);
     // He-uniform initialisation (host, seeded), zero biases; Adam state zero
     std::vector<float> w0(np, 0.f);
     std::mt19937_64 gen(seed);
@@ -909,14 +917,14 @@ static StepArgs step_args(bnm_mlp* p, int mode, int batch, const float* X, const
     return a;
 }
 
-static int launch_step(bnm_mlp* p, const StepArgs& a) {
+static int launch_step(bnm_mlp* p, const StepArgs& a, int clusters = 1) {
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof cfg);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)p->cluster;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)p->cluster);
+    cfg.gridDim = dim3((unsigned)(p->cluster * clusters));
     cfg.blockDim = dim3(kStepThreads);
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -950,7 +958,7 @@ extern "C" int bnm_mlp_predict(bnm_mlp* p, const float* X, int32_t n, float* Y) 
     for (int s = 0; s < n; s += p->max_batch) {
         const int B = std::min(p->max_batch, n - s);
         BNM_CUDA_TRY(cudaMemcpyAsync(p->xin, X + (size_t)s * p->in, (size_t)B * p->in * 4, cudaMemcpyHostToDevice, p->st));
-        int rc = launch_step(p, step_args(p, kForward, B, p->xin, nullptr));
+        int rc = launch_step(p, step_args(p, kForward, B, p->xin, nullptr), std::min(p->fwd_clusters, (B + 31) / 32));
         if (rc) return rc;
         BNM_CUDA_TRY(cudaMemcpyAsync(Y + (size_t)s * p->out, p->yout, (size_t)B * p->out * 4, cudaMemcpyDeviceToHost, p->st));
     }

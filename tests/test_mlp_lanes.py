@@ -1,6 +1,7 @@
-"""Training steps in which the lanes of a warp go different ways: gradients so
-small that some weights of a lane take Adam's plain expression, rows past the
-batch, layers whose last 32 outputs are not full (GPU)."""
+"""The surrogate's kernels off their usual path (GPU): training steps in which
+the lanes of a warp go different ways (gradients so small that some weights of a
+lane take Adam's plain expression, rows past the batch, layers whose last 32
+outputs are not full); forward passes over several clusters."""
 import numpy as np
 import pytest
 
@@ -33,3 +34,23 @@ def test_small_gradients_take_the_same_formula(n_in, hidden, layers, out):
     mm, v = (f(1) - b1) * g, (f(1) - b2) * g * g
     want = w - f(1e-2) * (mm / (f(1) - b1)) / (np.sqrt(v / (f(1) - b2)) + f(1e-8))
     np.testing.assert_array_equal(m.get_params(), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,max_batch", [(1, 1), (33, 1024), (300, 256), (1500, 1024)])
+def test_wide_forward_does_not_depend_on_the_split(n, max_batch):
+    """Networks too wide for the forward kernel's shared memory: rows in one or several clusters, odd blocks left
+    over; a row's result is what it gives alone."""
+    from oracle import mlp_oracle
+
+    n_in, hidden, layers, out = 21, 3300, 2, 3
+    m = S.MLP(n_in, out, hidden=hidden, layers=layers, max_batch=max_batch, seed=2)
+    X = np.random.default_rng(n).standard_normal((n, n_in)).astype(np.float32)
+    y = m.predict(X)
+    for i in sorted({0, n // 2, n - 1}):
+        np.testing.assert_array_equal(m.predict(X[i:i + 1])[0], y[i])
+    some = X[:40]
+    ref = mlp_oracle.loss_and_grads(m.get_params(), [n_in] + [hidden] * layers + [out], some,
+                                    np.zeros((len(some), out), np.float32))[2]
+    # the oracle rounds where the device does: what is left is FP32 summation and rare BF16 rounding flips
+    assert np.linalg.norm(y[:40] - ref) <= 1e-3 * np.linalg.norm(ref)
