@@ -733,8 +733,10 @@ struct bnm_mlp {
     void* slab = nullptr;  // the device buffers above, except the growing ones (data_x, data_y, idx)
 };
 
-// Training steps per launch: bounds the index buffer and the time one launch holds its SMs.
+// Training steps per launch, and row indices of those steps (16 MB): bound the
+// index buffer and the time one launch holds its SMs.
 static constexpr int kMaxSteps = 2048;
+static constexpr long long kMaxIdx = 4 << 20;
 
 extern "C" void bnm_mlp_destroy(bnm_mlp* p) {
     if (!p) return;
@@ -997,7 +999,8 @@ extern "C" int bnm_mlp_train(bnm_mlp* p, const float* X, const float* Y, int32_t
         p->data_n = n;
     }
     const long long total = (long long)nb * epochs;
-    const size_t need = (size_t)std::min<long long>(total, kMaxSteps) * batch;
+    const int max_steps = (int)std::max<long long>(1, std::min<long long>(kMaxSteps, kMaxIdx / batch));
+    const size_t need = (size_t)std::min<long long>(total, max_steps) * batch;
     if (p->idx_cap < need) {
         if (p->idx) cudaFree(p->idx);
         p->idx = nullptr;
@@ -1014,7 +1017,7 @@ extern "C" int bnm_mlp_train(bnm_mlp* p, const float* X, const float* Y, int32_t
     std::vector<float2> c12;
     std::vector<float> losses((size_t)total);
     long long done = 0;
-    // one launch per kMaxSteps steps
+    // one launch per max_steps steps
     auto flush = [&]() -> int {
         const int steps = (int)c12.size();
         if (!steps) return BNM_OK;
@@ -1043,7 +1046,7 @@ extern "C" int bnm_mlp_train(bnm_mlp* p, const float* X, const float* Y, int32_t
             idx.insert(idx.end(), order.begin() + (size_t)s * batch, order.begin() + (size_t)(s + 1) * batch);
             p->adam_t++;
             c12.push_back(make_float2(1.f - std::pow(b1, (float)p->adam_t), 1.f - std::pow(b2, (float)p->adam_t)));
-            if ((int)c12.size() == kMaxSteps && (rc = flush())) return rc;
+            if ((int)c12.size() == max_steps && (rc = flush())) return rc;
         }
     }
     if ((rc = flush())) return rc;

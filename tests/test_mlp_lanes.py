@@ -54,3 +54,23 @@ def test_wide_forward_does_not_depend_on_the_split(n, max_batch):
                                     np.zeros((len(some), out), np.float32))[2]
     # the oracle rounds where the device does: what is left is FP32 summation and rare BF16 rounding flips
     assert np.linalg.norm(y[:40] - ref) <= 1e-3 * np.linalg.norm(ref)
+
+
+@pytest.mark.gpu
+def test_long_trainings_of_large_batches_stay_in_bounded_memory():
+    """The rows of a launch's steps are bounded, whatever the batch: 150 steps of 65,536 rows are 37 MB of indices, of
+    which 16 are on the device at once; and where a training is cut into launches does not show in its result."""
+    import torch
+
+    n, epochs = 65536, 150
+    x, t = np.full((n, 2), 0.7, np.float32), np.full((n, 1), 0.3, np.float32)  # equal rows: their order does not matter
+    m = [S.MLP(2, 1, hidden=8, layers=1, max_batch=n, seed=7) for _ in range(2)]
+    for k in m:
+        k.fine_tune(x, t, epochs=1, batch=n, lr=1e-3)  # the training set is on the device
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    once = m[0].fine_tune(x, t, epochs=epochs, batch=n, lr=1e-3)
+    assert free - torch.cuda.mem_get_info()[0] <= 24 << 20
+    parts = np.concatenate([m[1].fine_tune(x, t, epochs=10, batch=n, lr=1e-3) for _ in range(epochs // 10)])
+    np.testing.assert_array_equal(once, parts)
+    np.testing.assert_array_equal(m[0].get_params(), m[1].get_params())
