@@ -1,7 +1,8 @@
 """The surrogate's kernels off their usual path (GPU): training steps in which
 the lanes of a warp go different ways (gradients so small that some weights of a
 lane take Adam's plain expression, rows past the batch, layers whose last 32
-outputs are not full); forward passes over several clusters."""
+outputs are not full); forward passes over several clusters; calls around the
+size of the locked buffer."""
 import numpy as np
 import pytest
 
@@ -74,3 +75,18 @@ def test_long_trainings_of_large_batches_stay_in_bounded_memory():
     parts = np.concatenate([m[1].fine_tune(x, t, epochs=10, batch=n, lr=1e-3) for _ in range(epochs // 10)])
     np.testing.assert_array_equal(once, parts)
     np.testing.assert_array_equal(m[0].get_params(), m[1].get_params())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_in,max_batch", [(4100, 96), (4100, 32), (19, 64)])
+def test_predict_around_the_locked_buffer(n_in, max_batch):
+    """1 MiB of rows: more than that goes through the device's buffer where it holds more (4100 inputs: 63 rows, so 48),
+    else in pieces; the buffer grows with the calls."""
+    rows = (1 << 20) // (4 * (n_in + 3)) // 16 * 16
+    m = S.MLP(n_in, 3, hidden=40, layers=1, max_batch=max_batch, seed=2)
+    X = np.random.default_rng(n_in).standard_normal((3 * rows + 5, n_in)).astype(np.float32)
+    y = m.predict(X)
+    for n in (1, 17, rows - 1, rows, rows + 1, 2 * rows + 7):
+        np.testing.assert_array_equal(m.predict(X[:n]), y[:n])
+    ref = np.concatenate([m.predict(X[i:i + 1]) for i in (0, rows, 3 * rows + 4)])
+    np.testing.assert_array_equal(y[[0, rows, 3 * rows + 4]], ref)
