@@ -656,9 +656,8 @@ __global__ void __launch_bounds__(kPredThreads) mlp_predict_kernel(const MlpLaye
 
 // One tile of a layer per warp, between the flat FP32 parameters and the
 // device's arrays: FP32 tiles and BF16 blocks from flat (pack), flat from the
-// tiles (unpack).  blockIdx.y: layer.
-__global__ void pack_kernel(const MlpLayer* layers, const float* flat, float4* w, float* bw) {
-    const MlpLayer& y = layers[blockIdx.y];
+// tiles (unpack).  blockIdx.y: layer, and those gridDim.y further on.
+__device__ __forceinline__ void pack_layer(const MlpLayer& y, const float* flat, float4* w, float* bw) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, ot = y.doutp / 16, ki = y.dinp / 16;
     const int warps = gridDim.x * (blockDim.x / 32), w0 = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     for (int k = w0; k < ot * (y.dinp / 8); k += warps) {
@@ -681,8 +680,11 @@ __global__ void pack_kernel(const MlpLayer* layers, const float* flat, float4* w
         bw[y.bias + o] = o < y.dout ? flat[y.boff + o] : 0.f;
 }
 
-__global__ void unpack_kernel(const MlpLayer* layers, const float4* w, const float* bw, float* flat) {
-    const MlpLayer& y = layers[blockIdx.y];
+__global__ void pack_kernel(const MlpLayer* layers, int L, const float* flat, float4* w, float* bw) {
+    for (int l = blockIdx.y; l < L; l += gridDim.y) pack_layer(layers[l], flat, w, bw);
+}
+
+__device__ __forceinline__ void unpack_layer(const MlpLayer& y, const float4* w, const float* bw, float* flat) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, ot = y.doutp / 16;
     const int warps = gridDim.x * (blockDim.x / 32), w0 = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     for (int k = w0; k < ot * (y.dinp / 8); k += warps) {
@@ -696,6 +698,9 @@ __global__ void unpack_kernel(const MlpLayer* layers, const float4* w, const flo
     }
     for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < y.dout; o += gridDim.x * blockDim.x)
         flat[y.boff + o] = bw[y.bias + o];
+}
+__global__ void unpack_kernel(const MlpLayer* layers, int L, const float4* w, const float* bw, float* flat) {
+    for (int l = blockIdx.y; l < L; l += gridDim.y) unpack_layer(layers[l], w, bw, flat);
 }
 
 int pad16(int x) { return (x + 15) / 16 * 16; }
@@ -760,9 +765,11 @@ extern "C" void bnm_mlp_destroy(bnm_mlp* p) {
     delete p;
 }
 
+static dim3 layer_grid(const bnm_mlp* p) { return dim3(64, (unsigned)std::min(p->L, 65535)); }  // the grid's limit
+
 // Device arrays from the flat parameters, Adam's state cleared (asynchronous)
 static cudaError_t load_flat(bnm_mlp* p) {
-    pack_kernel<<<dim3(64, p->L), 256, 0, p->st>>>(p->d_lay, p->flat, p->w, p->bw);
+    pack_kernel<<<layer_grid(p), 256, 0, p->st>>>(p->d_lay, p->L, p->flat, p->w, p->bw);
     cudaError_t e = cudaGetLastError();
     // m, v, bm, bv follow one another in the slab
     if (e == cudaSuccess)
@@ -1114,7 +1121,7 @@ extern "C" int64_t bnm_mlp_num_params(const bnm_mlp* p) { return p ? p->n_params
 extern "C" int bnm_mlp_get_params(bnm_mlp* p, float* flat) {
     if (!p || !flat) return bnm_fail_msg(BNM_EINVAL, "null argument");
     BNM_CUDA_TRY(cudaSetDevice(p->device));
-    unpack_kernel<<<dim3(64, p->L), 256, 0, p->st>>>(p->d_lay, p->w, p->bw, p->flat);
+    unpack_kernel<<<layer_grid(p), 256, 0, p->st>>>(p->d_lay, p->L, p->w, p->bw, p->flat);
     BNM_CUDA_TRY(cudaGetLastError());
     BNM_CUDA_TRY(cudaMemcpyAsync(flat, p->flat, (size_t)p->n_params * 4, cudaMemcpyDeviceToHost, p->st));
     BNM_CUDA_TRY(cudaStreamSynchronize(p->st));

@@ -90,3 +90,14 @@ def test_predict_around_the_locked_buffer(n_in, max_batch):
         np.testing.assert_array_equal(m.predict(X[:n]), y[:n])
     ref = np.concatenate([m.predict(X[i:i + 1]) for i in (0, rows, 3 * rows + 4)])
     np.testing.assert_array_equal(y[[0, rows, 3 * rows + 4]], ref)
+
+
+@pytest.mark.gpu
+def test_more_layers_than_a_grid_has_rows():
+    layers = 65600
+    m = S.MLP(1, 1, hidden=1, layers=layers, max_batch=1, seed=0)
+    w = np.tile(np.float32([1, 0]), layers + 1)  # every layer passes its input on
+    w[-1] = 0.25
+    m.set_params(w)
+    np.testing.assert_array_equal(m.get_params(), w)
+    np.testing.assert_array_equal(m.predict(np.float32([[1.5]])), np.float32([[1.75]]))
