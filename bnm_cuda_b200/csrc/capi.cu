@@ -285,19 +285,23 @@ static int plan_create(const bnm_config* cfg, const double* sc, const double* em
     p->pad = (cfg->precision == BNM_PREC_F32 && !p->kmax && (N & 1)) ? 1 : 0;
     p->sc_ld = p->kmax ? p->kmax : N + p->pad;
     std::vector<float> sc32((size_t)(N + p->pad) * p->sc_ld, 0.f);
-    std::vector<double> scfic((size_t)N * N), sc64((size_t)N * N);  // sc64: transposed
+    std::vector<double> scfic((size_t)N * N);
     for (int i = 0; i < N; i++)
         for (int j = 0; j < N; j++) {
             sc32[(size_t)i * p->sc_ld + j] = (float)sc[(size_t)i * N + j];
-            sc64[(size_t)j * N + i] = sc[(size_t)i * N + j];
             scfic[(size_t)i * N + j] =
                 cfg->precision == BNM_PREC_F32_REF ? (double)(float)sc[(size_t)i * N + j] : sc[(size_t)i * N + j];
         }
     BNM_CUDA_TRY(dalloc(p, &p->d_sc32, sc32.size()));
-    BNM_CUDA_TRY(dalloc(p, &p->d_sc64, (size_t)N * N));
     BNM_CUDA_TRY(dalloc(p, &p->d_sc_fic, (size_t)N * N));
     BNM_CUDA_TRY(cudaMemcpy(p->d_sc32, sc32.data(), sc32.size() * 4, cudaMemcpyHostToDevice));
-    BNM_CUDA_TRY(cudaMemcpy(p->d_sc64, sc64.data(), sc64.size() * 8, cudaMemcpyHostToDevice));
+    if (cfg->precision == BNM_PREC_F64) {  // by columns
+        std::vector<double> sc64((size_t)N * N);
+        for (int j = 0; j < N; j++)
+            for (int i = 0; i < N; i++) sc64[(size_t)j * N + i] = sc[(size_t)i * N + j];
+        BNM_CUDA_TRY(dalloc(p, &p->d_sc64, sc64.size()));
+        BNM_CUDA_TRY(cudaMemcpy(p->d_sc64, sc64.data(), sc64.size() * 8, cudaMemcpyHostToDevice));
+    }
     BNM_CUDA_TRY(cudaMemcpy(p->d_sc_fic, scfic.data(), scfic.size() * 8, cudaMemcpyHostToDevice));
 
     // noise: the caller's table (HOST), or Philox values.  The FP32 kernels can
