@@ -636,7 +636,8 @@ template <typename TB>
 static cudaError_t launch_fc_window(const FcArgs& a, const TB* bold, cudaStream_t st) {
     int ppt = a.ppt;
     if (!ppt) {
-        const long long ctas = (long long)a.P * a.n_sims / 256;  // of the smallest tile
+        // of the smallest tile; 300: two for each of the GPU's 148 SMs
+        const long long ctas = (long long)a.P * a.n_sims / 256;
         ppt = ctas >= 8 * 300 ? 8 : ctas >= 4 * 300 ? 4 : ctas >= 2 * 300 ? 2 : 1;
     }
     switch (ppt) {
@@ -681,7 +682,7 @@ cudaError_t bnm_launch_fcd(const FcdArgs& a, cudaStream_t st) {
         return side * (side + 1) / 2;
     };
     // The larger tile reads each row half as often and costs 2.5-2.8 of the
-    // smaller: it pays where there are two CTAs of it for each SM and the
+    // smaller: it pays where there are two CTAs of it for each SM (296) and the
     // windows do not leave much of it empty (W = 278, 15 tiles against 45, 64
     // simulations: 0.92 against 1.04 ms; W = 85, 3 against 6, 300 simulations:
     // 132 against 110 us; 60 tiles in all: 169 against 116 us).

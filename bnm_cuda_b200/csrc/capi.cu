@@ -1116,11 +1116,13 @@ static int read_timings(bnm_plan* p);
 // need about the same number of substeps.  In the register kernel a
 // particle that hits the numerical-FIC trial cap integrates about 1 M more
 // substeps than one that needs no restart, and with more particles than SMs
-// the CTAs share SMs (two per SM, each slower than alone), so the generation
+// the CTAs share SMs (as many per SM as it holds, each slower than alone), so the generation
 // ends with the heavy particles that shared an SM.  The kernel hands out
-// io_order from both ends: the second CTA on an SM takes the lightest
-// particles, every other CTA the heaviest, so heavy particles run alone or
-// beside light ones.  Work is predicted by the FIC restart count of the
+// io_order from both ends: the first CTA on an SM takes the heaviest particles,
+// all later ones the lightest, so heavy particles run alone or beside light
+// ones.  (30 s with FIC, on against off: N = 100, 256 particles 275 and 353 ms; with
+// three or more CTAs an SM N = 83, 450 particles 345 and 392, N = 60, 450 230 and 280,
+// N = 30, 1200 225 and 238.)  Work is predicted by the FIC restart count of the
 // nearest particle simulated before by this plan (G, mean wEE, mean wEI, each
 // scaled by its spread); io_order lists the particles heaviest first.
 // Without history (fewer than 16 particles) the order is the identity.  Where
@@ -1267,7 +1269,6 @@ extern "C" int bnm_run(bnm_plan* p, int32_t n, const double* G, const double* w_
     if (!p || !out || !G || !w_ee || !w_ei) return fail(BNM_EINVAL, "null argument");
     if (n < 1 || n > p->cfg.max_sims) return fail(BNM_EINVAL, "n=%d outside [1, max_sims=%d]", n, p->cfg.max_sims);
     const bnm_config& c = p->cfg;
-    const bnm_sizes& s = p->sz;
     const int N = c.nodes;
     if (!c.do_fic && !w_ie) return fail(BNM_EINVAL, "w_ie is required when do_fic == 0");
     BNM_CUDA_TRY(cudaSetDevice(c.device));
@@ -1405,7 +1406,6 @@ static int ensure_pinned(bnm_plan* p) {
 // stream operations only (capturable).  The integrator must be tuned.
 static int enqueue_run(bnm_plan* p, int n) {
     const bnm_config& c = p->cfg;
-    const bnm_sizes& s = p->sz;
     const int N = c.nodes;
     cudaStream_t st = p->st;
     int rc;
@@ -1558,9 +1558,9 @@ static int integrator_ctas(const IntegratorShape& s, int n, int num_sms) {
 // While the fastest shapes of all plans leave every CTA an SM of its own, the
 // plans do not take SMs from one another and the fastest shapes are kept;
 // otherwise each plan gets the shape with the least SM time.  (Two subjects
-// of 68 and 84 nodes, 32 particles each: by SM time the second ran two
-// particles per CTA on a GPU with 84 idle SMs, 543 ms a generation; 286 ms by
-// time.)
+// of 68 and 84 nodes, 32 particles each, on a GPU with 84 idle SMs: by SM time
+// the timing's noise could pick two particles per CTA for the second, 543 ms a
+// generation in such a run; 285 ms otherwise.)
 static int group_shapes(bnm_group* g) {
     const size_t np = g->plans.size();
     std::vector<IntegratorShape> share(np);

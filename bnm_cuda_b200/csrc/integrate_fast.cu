@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(128, 1) integrate_fast_kernel(SimArgs a) {
 //     hangs on one comparison each and lies out of line;
 //   * a CTA of one warp (N <= 32) needs no block barrier between substeps.
 // Integration alone, against integrate_fast_kernel: N = 10, 24 s 28.8 -> 26.9
-// ms; N = 30, 200 particles 32.4 -> 29.4; N = 68, 256 particles with FIC 223 ->
+// ms; N = 30, 200 particles 32.4 -> 29.0; N = 68, 256 particles with FIC 223 ->
 // 215; N = 84, 32 particles 42.2 -> 41.4.  At N = 100 the same code is slower
 // (256 particles, 120 s: 533 against 495 ms): the ten unrolled substeps and
 // their ends no longer fit the instruction cache, which also rules out longer
@@ -842,8 +842,9 @@ static int fast_resident(F* fn, int threads, size_t smem) {
 }
 
 // CTAs are persistent over the batch, as many as the GPU holds at once.  (For
-// 300 particles at N = 83, three CTAs an SM give 64 ms, as two at most did with
-// 4 particles in a second round: two CTAs fill an SM's issue slots.)
+// 300 particles at N = 83, three CTAs on 4 SMs give 64 ms, as two at most did
+// with 4 particles in a second round; either way the other SMs, with two, are
+// done after 40, the time of 296 particles.)
 // Kernel and shared memory of a variant: integrate_reg_kernel for one particle
 // per CTA with a noise table and N <= 96 (its comment has both sides of the
 // line), else integrate_fast_kernel.

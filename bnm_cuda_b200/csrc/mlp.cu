@@ -158,12 +158,16 @@ __device__ __forceinline__ void mma_tiles(int kb, float (&d)[nA * nB][4], F load
 // with every operation rounded to nearest.  The hardware has no FP32 division
 // or square root: CUDA's are subroutines with a branch each, which a warp goes
 // through one after the other (about 6000 cycles for the 8 parameters of a
-// lane).  Here the quotients and the root are formed in FP64 to a relative
-// error below 2^-51 and rounded to FP32, without branches, so the parameters'
-// chains interleave.  That gives the same FP32 values: a quotient of two
-// 24-bit numbers, or the root of one, is at least 2^-49 away (relative) from
-// the midpoint of two FP32 neighbours, unless the result is subnormal; lanes
-// with a value near those ranges take the plain expression.
+// lane).  Here the quotients and the root are formed in FP64, without branches,
+// so the parameters' chains interleave, and rounded to FP32.  That gives the
+// same FP32 values: a quotient of two 24-bit numbers is at least 2^-49 away
+// (relative) from the midpoint of two FP32 neighbours, and the root of one at
+// least 2^-51 (x - y^2, for a midpoint y, is an odd multiple of 2^-48 with x in
+// [1, 4), hence |sqrt(x) - y| / y > 2^-49 / x), unless the result is subnormal.
+// The FP64 errors are below that: two roundings, 2^-52, for the quotients by
+// rc1, rc2; the last step's rounding, 2^-53, plus what the Newton steps leave of
+// the 2^-22 estimates (less than 2^-60 for the root, 2^-88 for the quotient).
+// Lanes with a value near the ends of the range take the plain expression.
 __device__ __forceinline__ float adam_plain(float w, float m, float v, const StepArgs& a, float c1, float c2) {
     return w - a.lr * (m / c1) / (sqrtf(v / c2) + a.eps);
 }

@@ -166,7 +166,7 @@ int bnm_plan_graph(bnm_plan *plan, int32_t *graph_launched);
  * whose blocks take particles by index): the plan predicts each particle's FIC
  * restarts from the nearest of the last 4096 particles it simulated.  The
  * register integrator (N <= 128, noise table) gives the heaviest particles to
- * CTAs alone on an SM and the lightest to the second CTA of an SM; the
+ * the first CTA on each SM and the lightest to the CTAs that come after it; the
  * two-particle column-split clusters pair particles of similar predicted work.
  * Results do not depend on it.  enabled: the plan places particles
  * (BNM_B200_PLACE=0 at plan creation turns it off); placed_last: the last
